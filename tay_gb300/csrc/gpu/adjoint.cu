@@ -179,6 +179,7 @@ SeeLaunch see_launch(TgpuBatch *b, const KernelRun &r, const PassIO &io) {
     S.pairs = b->d_pairs;
     S.telemetry = nullptr;
     S.io = io;
+    S.lanes = r.walk_lanes;
     return S;
 }
 
@@ -296,11 +297,14 @@ void backward_step(TgpuAdjoint *a, const Record &r, const StepList *pl = nullptr
         // particle itself, which both adjoints skip)
         F.plist = PairList{pl->idx, pl->count, b->total, b->plist_cap, 2u, rd.d_radii, rd.d_see_ctx};
         D.plist = F.plist;
+        F.lanes = rf.replay_lanes;
+        D.lanes = rd.replay_lanes;
         a->K->force_adj_replay(F, 0, st);
     } else {
         if (b->plist_idx && rf.skip_self) {
             F.plist = PairList{b->plist_idx, b->plist_count, b->total, b->plist_cap, 1u, nullptr, nullptr};
             D.plist = PairList{b->plist_idx, b->plist_count, b->total, b->plist_cap, 2u, rf.d_radii, rf.d_see_ctx};
+            D.lanes = rd.replay_lanes;
         }
         a->K->force_adj(F, 0, st);
     }

@@ -93,10 +93,34 @@ const ModelDesc *model_boids();
 const ModelDesc *model_sph();
 const ModelDesc *model_box();
 
+// See pass with G lanes per seer (see_group_kernel), for passes with terms; returns whether
+// it stored the records through L.wt.
+template <class P, int G>
+bool launch_group_t(const SeeLaunch &L, cudaStream_t st) {
+    if constexpr (see_detail::TermsOf<P>::value) {
+        if constexpr (!std::is_void_v<typename see_detail::CodecOf<P>::type>) {
+            if (L.wt) {
+                see_group_kernel<P, G, true><<<L.ctas * G, kSeeThreads, 0, st>>>(L);
+                return true;
+            }
+        }
+        see_group_kernel<P, G><<<L.ctas * G, kSeeThreads, 0, st>>>(L);
+    }
+    return false;
+}
+
 // helpers used by the model translation units
 template <class P>
 bool launch_see_t(const SeeLaunch &L, size_t smem, cudaStream_t st) {
     if (!L.ctas) return L.wt != nullptr;  // nothing to write
+    if (see_detail::TermsOf<P>::value && L.rows && !L.stage_cap && !L.hit_masks && L.union_factor <= 1) {
+        switch (L.lanes) {
+            case 8: return launch_group_t<P, 8>(L, st);
+            case 16: return launch_group_t<P, 16>(L, st);
+            case 32: return launch_group_t<P, 32>(L, st);
+            default: break;
+        }
+    }
     // the row kernel with the warp-union and hit-mask walks only when a tuning asks for them
     const bool warp_walks = L.hit_masks || L.union_factor > 1;
     if constexpr (!std::is_void_v<typename see_detail::CodecOf<P>::type>) {

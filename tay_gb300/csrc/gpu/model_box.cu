@@ -35,14 +35,34 @@ struct Seer {
     float4 mx, v, f;
 };
 
-// test/agent.c:57-63: b_buffer += b.min - a.min; b_buffer_count++
-template <class Acc>
-TGPU_D void see_fn(Seer &s, const float4 &a, const float4 &b, const Acc &, uint32_t, const SeeCtx &) {
-    s.bx = s.bx + (b.x - a.x);
-    s.by = s.by + (b.y - a.y);
-    s.bz = s.bz + (b.z - a.z);
+// test/agent.c:57-63: b_buffer += b.min - a.min; b_buffer_count++ (the pair's term, and its sum)
+struct Term {
+    float x, y, z;
+};
+TGPU_D void fold_fn(Seer &s, const Term &t) {
+    s.bx = s.bx + t.x;
+    s.by = s.by + t.y;
+    s.bz = s.bz + t.z;
     s.count += 1;
 }
+struct See {
+    using Term = box::Term;
+    static constexpr bool kCheapTerm = true;
+    static constexpr bool kSeenMinusSeer = true;  // d = b - a
+    template <class Acc>
+    TGPU_D static bool term(const Seer &, const float4 &a, const float4 &b, const Acc &, uint32_t, const SeeCtx &,
+                            Term &t) {
+        t = {b.x - a.x, b.y - a.y, b.z - a.z};
+        return true;
+    }
+    TGPU_D static void fold(Seer &s, const Term &t, const SeeCtx &) { fold_fn(s, t); }
+    template <class Acc>
+    TGPU_D static void see(Seer &s, const float4 &a, const float4 &b, const Acc &acc, uint32_t j, const SeeCtx &c) {
+        Term t;
+        term(s, a, b, acc, j, c, t);
+        fold_fn(s, t);
+    }
+};
 
 // test/agent.c:65-118 on registers: fold, move both corners, then the walls in the order
 // min x, y, z, max x, y, z.
@@ -75,7 +95,7 @@ TGPU_D void act_fn(float4 &mn, float4 &mx, float4 &v, float &bx, float &by, floa
 
 struct Codec;  // the record codec, defined below
 
-struct SeeOnly {
+struct SeeOnly : See {
     using SeeCtx = box::SeeCtx;
     using Codec = box::Codec;
     using ActCtx = box::SeeCtx;
@@ -90,16 +110,12 @@ struct SeeOnly {
         s.bz = b.z;
         s.count = __float_as_int(b.w);
     }
-    template <class Acc>
-    TGPU_D static void see(Seer &s, const float4 &a, const float4 &b, const Acc &acc, uint32_t j, const SeeCtx &c) {
-        see_fn(s, a, b, acc, j, c);
-    }
     TGPU_D static void finish(Seer &s, const float4 &, const PassIO &io, uint32_t i, const SeeCtx &, const ActCtx &) {
         io.out_f4[BBUF][i] = make_float4(s.bx, s.by, s.bz, __int_as_float(s.count));
     }
 };
 
-struct SeeAct {
+struct SeeAct : See {
     using SeeCtx = box::SeeCtx;
     using Codec = box::Codec;
     using ActCtx = box::ActCtx;
@@ -116,10 +132,6 @@ struct SeeAct {
         s.mx = io.in_f4[MAX][i];
         s.v = io.in_f4[VEL][i];
         s.f = io.in_f4[FBUF][i];
-    }
-    template <class Acc>
-    TGPU_D static void see(Seer &s, const float4 &a, const float4 &b, const Acc &acc, uint32_t j, const SeeCtx &c) {
-        see_fn(s, a, b, acc, j, c);
     }
     TGPU_D static void finish(Seer &s, const float4 &a, const PassIO &io, uint32_t i, const SeeCtx &,
                               const ActCtx &c) {

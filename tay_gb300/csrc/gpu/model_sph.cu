@@ -103,13 +103,22 @@ struct Density {
         return dist2(a.x - b.x, a.y - b.y, a.z - b.z) < c.support2;
     }
     TGPU_D static void load(Seer &s, const PassIO &, uint32_t, const Ctx &, const Ctx &) { s.rho = 0.0f; }
+    struct Term {
+        float w;
+    };
     template <class Acc>
-    TGPU_D static void see(Seer &s, const float4 &a, const float4 &b, const Acc &, uint32_t, const Ctx &c) {
+    TGPU_D static bool term(const Seer &, const float4 &a, const float4 &b, const Acc &, uint32_t, const Ctx &c,
+                            Term &t) {
         const float r2 = dist2(a.x - b.x, a.y - b.y, a.z - b.z);
-        if (r2 < c.support2) {
-            const float q = __fsqrt_rn(r2) * c.inv_h;
-            s.rho = __fmaf_rn(c.m, kernel_w(q, c.sigma), s.rho);
-        }
+        if (!(r2 < c.support2)) return false;
+        t.w = kernel_w(__fsqrt_rn(r2) * c.inv_h, c.sigma);
+        return true;
+    }
+    TGPU_D static void fold(Seer &s, const Term &t, const Ctx &c) { s.rho = __fmaf_rn(c.m, t.w, s.rho); }
+    template <class Acc>
+    TGPU_D static void see(Seer &s, const float4 &a, const float4 &b, const Acc &acc, uint32_t j, const Ctx &c) {
+        Term t;
+        if (term(s, a, b, acc, j, c, t)) fold(s, t, c);
     }
     TGPU_D static void finish(Seer &s, const float4 &, const PassIO &io, uint32_t i, const Ctx &c, const Ctx &) {
         const float P = kPressure ? pressure(s.rho, c) : 0.0f;
@@ -153,31 +162,45 @@ struct Force {
         s.A = rp.z;
         s.v = io.in_f4[VEL][i];
     }
+    struct __align__(16) Term {
+        float coef, dx, dy, dz;
+    };
     template <class Acc>
-    TGPU_D static void see(Seer &s, const float4 &a, const float4 &b, const Acc &acc, uint32_t j, const Ctx &c) {
+    TGPU_D static bool term(const Seer &s, const float4 &a, const float4 &b, const Acc &acc, uint32_t j, const Ctx &c,
+                            Term &t) {
         const float dx = a.x - b.x, dy = a.y - b.y, dz = a.z - b.z;
         const float r2 = dist2(dx, dy, dz);
-        if (r2 < c.support2 && r2 > 0.0f) {
-            const float4 bv = acc.f4(1, j);
-            const float4 brp = acc.f4(2, j);
-            // 1/r from one correctly rounded reciprocal square root, r = r2 * (1/r), dw / r
-            // as a product, and the viscosity term's two divisions as one
-            const float inv_r = __frsqrt_rn(r2);
-            const float r = r2 * inv_r;
-            const float q = r * c.inv_h;
-            const float dw = kernel_dw(q, c.sigma, c.inv_h);
-            const float vx = s.v.x - bv.x, vy = s.v.y - bv.y, vz = s.v.z - bv.z;
-            const float vr = __fmaf_rn(vz, dz, __fmaf_rn(vy, dy, vx * dx));
-            float visc = 0.0f;
-            if (vr < 0.0f) {
-                const float rho_bar = 0.5f * (s.rho + brp.x);
-                visc = -(c.alpha * c.c0 * (c.h * vr)) / ((r2 + c.eta2) * rho_bar);
-            }
-            const float coef = -c.m * ((s.A + brp.z) + visc) * (dw * inv_r);
-            s.ax = __fmaf_rn(coef, dx, s.ax);
-            s.ay = __fmaf_rn(coef, dy, s.ay);
-            s.az = __fmaf_rn(coef, dz, s.az);
+        if (!(r2 < c.support2 && r2 > 0.0f)) return false;
+        const float4 bv = acc.f4(1, j);
+        const float4 brp = acc.f4(2, j);
+        // 1/r from one correctly rounded reciprocal square root, r = r2 * (1/r), dw / r
+        // as a product, and the viscosity term's two divisions as one
+        const float inv_r = __frsqrt_rn(r2);
+        const float r = r2 * inv_r;
+        const float q = r * c.inv_h;
+        const float dw = kernel_dw(q, c.sigma, c.inv_h);
+        const float vx = s.v.x - bv.x, vy = s.v.y - bv.y, vz = s.v.z - bv.z;
+        const float vr = __fmaf_rn(vz, dz, __fmaf_rn(vy, dy, vx * dx));
+        float visc = 0.0f;
+        if (vr < 0.0f) {
+            const float rho_bar = 0.5f * (s.rho + brp.x);
+            visc = -(c.alpha * c.c0 * (c.h * vr)) / ((r2 + c.eta2) * rho_bar);
         }
+        t.coef = -c.m * ((s.A + brp.z) + visc) * (dw * inv_r);
+        t.dx = dx;
+        t.dy = dy;
+        t.dz = dz;
+        return true;
+    }
+    TGPU_D static void fold(Seer &s, const Term &t, const Ctx &) {
+        s.ax = __fmaf_rn(t.coef, t.dx, s.ax);
+        s.ay = __fmaf_rn(t.coef, t.dy, s.ay);
+        s.az = __fmaf_rn(t.coef, t.dz, s.az);
+    }
+    template <class Acc>
+    TGPU_D static void see(Seer &s, const float4 &a, const float4 &b, const Acc &acc, uint32_t j, const Ctx &c) {
+        Term t;
+        if (term(s, a, b, acc, j, c, t)) fold(s, t, c);
     }
     TGPU_D static void finish(Seer &s, const float4 &a, const PassIO &io, uint32_t i, const Ctx &, const Ctx &c) {
         if (!kIntegrate || kStoreAcc) io.out_f4[ACC][i] = make_float4(s.ax, s.ay, s.az, 0.0f);
@@ -336,11 +359,18 @@ struct ForceAdj {
         s.vb[0] = s.vb[1] = s.vb[2] = 0.0f;
         s.rhob = s.Pb = s.ta = s.tc = 0.0f;
     }
+    struct __align__(16) Term {
+        float xw[3];         // xbar's increments
+        float xwv, d[3];     // vbar's: xwv * d
+        float xmD, rb;       // Pbar's xmD; rhobar's xmD * rb
+        float ad, al, c0;    // theta's: ad * (al, c0)
+    };
     template <class Acc>
-    TGPU_D static void see(Seer &s, const float4 &a, const float4 &b, const Acc &acc, uint32_t j, const Ctx &c) {
+    TGPU_D static bool term(const Seer &s, const float4 &a, const float4 &b, const Acc &acc, uint32_t j, const Ctx &c,
+                            Term &t) {
         const float dx = a.x - b.x, dy = a.y - b.y, dz = a.z - b.z;
         const float r2 = dist2(dx, dy, dz);
-        if (!(r2 < c.support2 && r2 > 0.0f)) return;
+        if (!(r2 < c.support2 && r2 > 0.0f)) return false;
         const float4 bv = acc.f4(1, j), brp = acc.f4(2, j), bab = acc.f4(3, j);
         const float rinv = rsqrtf(r2);
         const float r = __fmul_rn(r2, rinv);
@@ -375,15 +405,32 @@ struct ForceAdj {
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
             const float inner = __fmaf_rn(coef_d, dd[k], __fmul_rn(coef_v, vv[k]));
-            s.xb[k] = __fadd_rn(s.xb[k], __fmaf_rn(xw, inner, __fmul_rn(cc, ww[k])));
-            s.vb[k] = __fmaf_rn(xwv, dd[k], s.vb[k]);
+            t.xw[k] = __fmaf_rn(xw, inner, __fmul_rn(cc, ww[k]));
+            t.d[k] = dd[k];
         }
-        const float xmD = __fmul_rn(xw, mD);
-        s.rhob = __fmaf_rn(xmD, __fmaf_rn(0.5f, Pi_rb, s.drho_A), s.rhob);
-        s.Pb = __fadd_rn(s.Pb, xmD);
-        const float ad = __fmul_rn(__fmaf_rn(s.ab.z, dz, __fmaf_rn(s.ab.y, dy, __fmul_rn(s.ab.x, dx))), mD);
-        s.ta = __fmaf_rn(ad, Pi_al, s.ta);
-        s.tc = __fmaf_rn(ad, Pi_c0, s.tc);
+        t.xwv = xwv;
+        t.xmD = __fmul_rn(xw, mD);
+        t.rb = __fmaf_rn(0.5f, Pi_rb, s.drho_A);
+        t.ad = __fmul_rn(__fmaf_rn(s.ab.z, dz, __fmaf_rn(s.ab.y, dy, __fmul_rn(s.ab.x, dx))), mD);
+        t.al = Pi_al;
+        t.c0 = Pi_c0;
+        return true;
+    }
+    TGPU_D static void fold(Seer &s, const Term &t, const Ctx &) {
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            s.xb[k] = __fadd_rn(s.xb[k], t.xw[k]);
+            s.vb[k] = __fmaf_rn(t.xwv, t.d[k], s.vb[k]);
+        }
+        s.rhob = __fmaf_rn(t.xmD, t.rb, s.rhob);
+        s.Pb = __fadd_rn(s.Pb, t.xmD);
+        s.ta = __fmaf_rn(t.ad, t.al, s.ta);
+        s.tc = __fmaf_rn(t.ad, t.c0, s.tc);
+    }
+    template <class Acc>
+    TGPU_D static void see(Seer &s, const float4 &a, const float4 &b, const Acc &acc, uint32_t j, const Ctx &c) {
+        Term t;
+        if (term(s, a, b, acc, j, c, t)) fold(s, t, c);
     }
     TGPU_D static void finish(Seer &s, const float4 &, const PassIO &io, uint32_t i, const Ctx &c, const Ctx &) {
         s.Pb *= s.inv_rho2;  // dc/dP_k = -m D / rho_k^2
@@ -434,16 +481,31 @@ struct DensityAdj {
         s.rhob = io.in_f4[A_RHOBAR][i].x;
         s.xb[0] = s.xb[1] = s.xb[2] = 0.0f;
     }
+    struct __align__(16) Term {
+        float g, dx, dy, dz;
+    };
     template <class Acc>
-    TGPU_D static void see(Seer &s, const float4 &a, const float4 &b, const Acc &acc, uint32_t j, const Ctx &c) {
+    TGPU_D static bool term(const Seer &s, const float4 &a, const float4 &b, const Acc &acc, uint32_t j, const Ctx &c,
+                            Term &t) {
         const float dx = a.x - b.x, dy = a.y - b.y, dz = a.z - b.z;
         const float r2 = dist2(dx, dy, dz);
-        if (!(r2 < c.support2 && r2 > 0.0f)) return;
+        if (!(r2 < c.support2 && r2 > 0.0f)) return false;
         const float rinv = rsqrtf(r2);
-        const float g = (s.rhob + acc.f4(1, j).x) * c.m * kernel_dw(r2 * rinv * c.inv_h, c.sigma, c.inv_h) * rinv;
-        s.xb[0] = __fmaf_rn(g, dx, s.xb[0]);
-        s.xb[1] = __fmaf_rn(g, dy, s.xb[1]);
-        s.xb[2] = __fmaf_rn(g, dz, s.xb[2]);
+        t.g = (s.rhob + acc.f4(1, j).x) * c.m * kernel_dw(r2 * rinv * c.inv_h, c.sigma, c.inv_h) * rinv;
+        t.dx = dx;
+        t.dy = dy;
+        t.dz = dz;
+        return true;
+    }
+    TGPU_D static void fold(Seer &s, const Term &t, const Ctx &) {
+        s.xb[0] = __fmaf_rn(t.g, t.dx, s.xb[0]);
+        s.xb[1] = __fmaf_rn(t.g, t.dy, s.xb[1]);
+        s.xb[2] = __fmaf_rn(t.g, t.dz, s.xb[2]);
+    }
+    template <class Acc>
+    TGPU_D static void see(Seer &s, const float4 &a, const float4 &b, const Acc &acc, uint32_t j, const Ctx &c) {
+        Term t;
+        if (term(s, a, b, acc, j, c, t)) fold(s, t, c);
     }
     TGPU_D static void finish(Seer &s, const float4 &, const PassIO &io, uint32_t i, const Ctx &, const Ctx &) {
         const float4 xb = io.in_f4[A_XBAR][i];

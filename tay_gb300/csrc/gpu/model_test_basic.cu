@@ -32,14 +32,34 @@ struct Seer {
     float4 v, f;
 };
 
-// test/agent.c:2-8: b_buffer += b.p - a.p; b_buffer_count++
-template <class Acc>
-TGPU_D void see_fn(Seer &s, const float4 &a, const float4 &b, const Acc &, uint32_t, const SeeCtx &) {
-    s.bx = s.bx + (b.x - a.x);
-    s.by = s.by + (b.y - a.y);
-    s.bz = s.bz + (b.z - a.z);
+// test/agent.c:2-8: b_buffer += b.p - a.p; b_buffer_count++ (the pair's term, and its sum)
+struct Term {
+    float x, y, z;
+};
+TGPU_D void fold_fn(Seer &s, const Term &t) {
+    s.bx = s.bx + t.x;
+    s.by = s.by + t.y;
+    s.bz = s.bz + t.z;
     s.count += 1;
 }
+struct See {
+    using Term = test_basic::Term;
+    static constexpr bool kCheapTerm = true;
+    static constexpr bool kSeenMinusSeer = true;  // d = b - a
+    template <class Acc>
+    TGPU_D static bool term(const Seer &, const float4 &a, const float4 &b, const Acc &, uint32_t, const SeeCtx &,
+                            Term &t) {
+        t = {b.x - a.x, b.y - a.y, b.z - a.z};
+        return true;
+    }
+    TGPU_D static void fold(Seer &s, const Term &t, const SeeCtx &) { fold_fn(s, t); }
+    template <class Acc>
+    TGPU_D static void see(Seer &s, const float4 &a, const float4 &b, const Acc &acc, uint32_t j, const SeeCtx &c) {
+        Term t;
+        term(s, a, b, acc, j, c, t);
+        fold_fn(s, t);
+    }
+};
 
 // test/agent.c:10-55 on registers
 TGPU_D void act_fn(float4 &p, float4 &v, float &bx, float &by, float &bz, int &count, float4 &f, const ActCtx &c) {
@@ -66,7 +86,7 @@ TGPU_D void act_fn(float4 &p, float4 &v, float &bx, float &by, float &bz, int &c
 
 struct Codec;  // the record codec, defined below
 
-struct SeeOnly {
+struct SeeOnly : See {
     using SeeCtx = test_basic::SeeCtx;
     using Codec = test_basic::Codec;
     using ActCtx = test_basic::SeeCtx;
@@ -80,16 +100,12 @@ struct SeeOnly {
         s.bz = b.z;
         s.count = __float_as_int(b.w);
     }
-    template <class Acc>
-    TGPU_D static void see(Seer &s, const float4 &a, const float4 &b, const Acc &acc, uint32_t j, const SeeCtx &c) {
-        see_fn(s, a, b, acc, j, c);
-    }
     TGPU_D static void finish(Seer &s, const float4 &, const PassIO &io, uint32_t i, const SeeCtx &, const ActCtx &) {
         io.out_f4[BBUF][i] = make_float4(s.bx, s.by, s.bz, __int_as_float(s.count));
     }
 };
 
-struct SeeAct {
+struct SeeAct : See {
     using SeeCtx = test_basic::SeeCtx;
     using Codec = test_basic::Codec;
     using ActCtx = test_basic::ActCtx;
@@ -104,10 +120,6 @@ struct SeeAct {
         s.count = __float_as_int(b.w);
         s.v = io.in_f4[VEL][i];
         s.f = io.in_f4[FBUF][i];
-    }
-    template <class Acc>
-    TGPU_D static void see(Seer &s, const float4 &a, const float4 &b, const Acc &acc, uint32_t j, const SeeCtx &c) {
-        see_fn(s, a, b, acc, j, c);
     }
     TGPU_D static void finish(Seer &s, const float4 &a, const PassIO &io, uint32_t i, const SeeCtx &,
                               const ActCtx &c) {

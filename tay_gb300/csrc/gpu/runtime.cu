@@ -242,6 +242,66 @@ int upload_contexts(TgpuBatch *b, int seg) {
     return TGPU_OK;
 }
 
+// Lanes per seer of a see pass over `seers` seers (row order).  With one lane per seer a
+// launch takes at least as long as one lane's walk, and needs enough seers to hide the
+// latency of its loads; below that the chip idles and several lanes share a seer's candidates
+// (see_group_kernel, which issues more instructions per candidate).  The longer a walk, the
+// more seers it takes: `mates` is the number of box-test passes a seer can expect from the
+// seen agents' mean density, and the size up to which 8 lanes win grows with about its cube
+// root.  Measured, us at 1 / 8 / 16 / 32 lanes, see pass (step where marked):
+//   SPH density, 512 mates:  2,048 seers 258 / 65 / 35 / 19, 20,480 433 / 129 / 98 / 84,
+//                            81,920 527 / 386 / 346 / 322, 262,144 1140 / 1162 / 1106 / 1062
+//   SPH force, list replay:  2,048 126 / 33 / 23 / 16, 20,480 147 / 57 / 56 / 67,
+//                            81,920 182 / 159 / 179 / 245, 131,072 233 / 264 / 298 / 400
+//   test model, 100 mates:   2,000 43 / 21 / 16 / 12, 12,000 53 / 24 / 26 / 33,
+//                            30,000 58 / 43 / 45 / 65, 50,000 62 / 63 / 71 / 102
+//   the same (step):  50 mates: 10,000 63 / 47 / 47 / 57, 40,000 72 / 70 / 83 / 117
+//                     25 mates: 5,000 53 / 43 / 43 / 48, 20,000 57 / 51 / 59 / 78, 40,000 61 / 65 / 81 / 116
+//                      4 mates: 10,000 49 / 45 / 49 / 59, 20,000 57 / 58 / 67 / 85
+//   two groups on a plane (step), 25 mates: 8,000 + 10,000 94 / 78 / 93 / 127, 16,000 each
+//                     97 / 92 / 122 / 179, 20,000 + 30,000 99 / 115 / 158 / 248
+uint32_t seer_lanes(uint64_t seers, double mates, int dims, bool replay) {
+    const double most = 9000.0 * pow(std::max(mates, 1.0), 0.37) * (dims < 3 ? 0.6 : 1.0);
+    if ((double)seers > most) return 1u;
+    if ((double)seers > most / 4.0) return 8u;
+    // a dense walk keeps 32 lanes busy row by row; a list of the same seer is shorter
+    if (mates >= 200.0 && !replay) return 32u;
+    return (double)seers > most / 16.0 ? 16u : 32u;
+}
+
+// The box-test passes an agent can expect among the agents of group `seen` if they were
+// spread evenly over their pushed extent (or fixed box).
+double expected_mates(const TgpuBatch *b, int seen, const float *radii) {
+    const HostSeg &h = b->hs[seen];
+    double mates = b->specs[seen].count;
+    for (int a = 0; a < seg_dims(b->specs[seen]); ++a) {
+        const double ext = h.g.box_fixed ? (double)h.g.box_max[a] - h.g.box_min[a] : (double)h.host_max[a] - h.host_min[a];
+        if (ext > 2.0 * radii[a]) mates *= 2.0 * radii[a] / ext;
+    }
+    return mates;
+}
+
+void set_lanes(TgpuBatch *b) {
+    for (auto &r : b->runs) {
+        if (!r.k->see) continue;
+        uint64_t seers = 0;
+        double mates = 0.0;
+        int dims = 3;
+        if (r.seer_seg >= 0) {
+            seers = b->specs[r.seer_seg].count;
+            dims = std::min(seg_dims(b->specs[r.seer_seg]), seg_dims(b->specs[r.seen_seg]));
+            mates = expected_mates(b, r.seen_seg, b->state_passes[r.see_pass].pass.radii);
+        } else {
+            seers = b->total;
+            dims = seg_dims(b->specs[0]);
+            for (int s = 0; s < b->nseg; ++s)
+                mates += expected_mates(b, s, b->hs[s].passes[r.see_pass].radii) * ((double)b->specs[s].count / std::max(b->total, 1u));
+        }
+        r.walk_lanes = seer_lanes(seers, mates, dims, false);
+        r.replay_lanes = seer_lanes(seers, mates, dims, true);
+    }
+}
+
 // Per-segment grid bounds from the pushed agents: each axis gets a power-of-two cell
 // budget with 10% headroom over the pushed extent (bounded to 1024, the 10-bit Morton
 // limit); the dense table gets at most shared_megabytes of uint2 entries.
@@ -250,6 +310,7 @@ int upload_contexts(TgpuBatch *b, int seg) {
 int tgpu::prepare_specs(TgpuBatch *b) {
     if (!b->specs_dirty) return TGPU_OK;
     b->specs_dirty = false;
+    set_lanes(b);
     std::vector<SegmentSpec> next = b->specs;
     uint64_t table_total = 0;
     uint32_t max_key_bits = 3;
@@ -403,6 +464,7 @@ void tgpu::attach_pair_list(const TgpuBatch *b, const KernelRun &r, SeeLaunch &S
     if (r.list_mode == 2u) {
         S.plist.rec_radii = b->runs[r.list_src].d_radii;
         S.plist.rec_ctx = b->runs[r.list_src].d_see_ctx;
+        S.lanes = r.replay_lanes;
     }
 }
 
@@ -476,6 +538,7 @@ void tgpu::enqueue_step(TgpuBatch *b, const StepEvents *E, bool write_through) {
             S.pairs = b->d_pairs;
             S.telemetry = b->d_telemetry;
             S.io = io;
+            S.lanes = r.walk_lanes;
             attach_pair_list(b, r, S);
             // Write-through on the final pass over every segment: each CTA stores its seers'
             // finished records to the host as it ends, so the host link overlaps the pass.

@@ -31,6 +31,7 @@ struct KernelRun {
     int seen_seg = -1;  // state batches: the segment whose agents a see pass reads
     uint32_t list_mode = 0;  // pair list (PairList): 0 none, 1 record, 2 replay
     int list_src = -1;       // replay: the run that records the list
+    uint32_t walk_lanes = 1, replay_lanes = 1;  // lanes per seer when the pass walks / replays
 };
 
 struct HostSeg {

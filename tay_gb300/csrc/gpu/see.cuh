@@ -443,15 +443,16 @@ struct CodecOf<P, std::void_t<typename P::Codec>> {
 // Write-through epilogue of a see CTA: its seers' finished records (the streams this
 // launch wrote, the others as they are) in the model's AoS layout, staged in shared
 // memory and stored to the segment's page-locked host records with 16-byte stores, so
-// the host link works while the rest of the pass runs.  Every thread of the CTA calls it.
-template <class C>
+// the host link works while the rest of the pass runs.  Every thread of the CTA calls it;
+// kSeers seers a CTA, one record each by its first threads.
+template <class C, uint32_t kSeers = (uint32_t)kSeeThreads>
 TGPU_D void write_through_cta(const SeeLaunch &L, uint32_t *wt, uint32_t first, uint32_t seg_begin,
                               uint32_t seg_end, uint32_t *sm) {
     constexpr uint32_t W = C::kAgentBytes / 4;
     PassIO wio = L.io;
 #pragma unroll
     for (int c = 0; c < kMaxF4; ++c) wio.in_f4[c] = wio.out_f4[c];
-    const uint32_t cnt = min((uint32_t)kSeeThreads, seg_end - first);
+    const uint32_t cnt = min(kSeers, seg_end - first);
     if (threadIdx.x < cnt) C::unpack(sm + threadIdx.x * W, wio, first + threadIdx.x, L.wt_program);
     __syncthreads();
     uint32_t *dst = wt + (size_t)(first - seg_begin) * W;
@@ -974,6 +975,348 @@ __global__ void __launch_bounds__(kSeeThreads, kStage ? 1 : 8) see_rows_kernel(S
         __shared__ __align__(16) uint32_t wt_sm[kSeeThreads * (C::kAgentBytes / 4)];
         uint32_t *wt = L.wt[seg];
         if (wt) write_through_cta<C>(L, wt, cta.y, S.begin, seg_end, wt_sm);
+    }
+}
+
+// ------------------------------------------------------------------ several lanes per seer
+
+namespace see_detail {
+
+// Whether pass P splits its see function into a term that depends on the pair alone and a
+// fold that adds it to the seer (P::Term, P::term, P::fold).
+template <class P, class = void>
+struct TermsOf {
+    static constexpr bool value = false;
+};
+template <class P>
+struct TermsOf<P, std::void_t<typename P::Term>> {
+    static constexpr bool value = true;
+};
+
+// Whether P's terms cost next to nothing and read nothing but the position (P::kCheapTerm):
+// they are computed where a candidate is tested.  Others are computed for the candidates that
+// passed, gathered until they fill the lanes.
+template <class P, class = void>
+struct CheapOf {
+    static constexpr bool value = false;
+};
+template <class P>
+struct CheapOf<P, decltype((void)P::kCheapTerm)> {
+    static constexpr bool value = P::kCheapTerm;
+};
+
+// Slots of a seer's queue: two chunks add at most 2 G to what the last ones left.
+constexpr int group_slots(int g) { return g > 8 ? 4 * g : 32; }
+
+// The G lanes of one seer, as a part of their warp (every lane of the warp calls the methods).
+template <int G>
+struct Group {
+    uint32_t shift, below;  // the group's first lane; the lanes of it below this one
+    TGPU_D explicit Group(uint32_t lane) : shift(lane & ~(uint32_t)(G - 1)), below((1u << (lane & (G - 1))) - 1u) {}
+    // The group's lanes with `p`, as bits 0..G-1.
+    TGPU_D uint32_t votes(bool p) const {
+        const uint32_t bits = __ballot_sync(0xffffffffu, p) >> shift;
+        return G == 32 ? bits : bits & ((1u << (G & 31)) - 1u);
+    }
+};
+
+// Folds a seer's first n <= kMost terms, in order (all its lanes hold the same seer and do the
+// same).
+template <class P, int kMost>
+TGPU_D void fold_terms(typename P::Seer &s, const typename P::Term *q, uint32_t n, const typename P::SeeCtx &c) {
+    __syncwarp();
+    if (__all_sync(0xffffffffu, n == (uint32_t)kMost)) {
+#pragma unroll
+        for (int k = 0; k < kMost; ++k) P::fold(s, q[k], c);
+    } else {
+        for (uint32_t k = 0; k < n; ++k) P::fold(s, q[k], c);
+    }
+    __syncwarp();
+}
+
+// The terms of up to G candidates of a seer, one a lane (those with `take`), folded in lane
+// order.
+template <class P, int G, class Acc>
+TGPU_D void eval_terms(typename P::Seer &s, const float4 &sp, bool take, uint32_t j, const float4 *pos,
+                       const Acc &acc, typename P::Term *q, const Group<G> &gr, const typename P::SeeCtx &c) {
+    typename P::Term t;
+    if (take) take = P::term(s, sp, __ldg(pos + j), acc, j, c, t);
+    const uint32_t v = gr.votes(take);
+    if (take) q[__popc(v & gr.below)] = t;
+    fold_terms<P, G>(s, q, (uint32_t)__popc(v), c);
+}
+
+// The box test without branches, on the difference the pass's own functions compute.
+template <class P>
+TGPU_D bool box_hit_flat(const float4 &a, const float4 &b, const float4 &r) {
+    constexpr bool kSeenFirst = SeenMinusSeerOf<P>::value;
+    const float dx = kSeenFirst ? b.x - a.x : a.x - b.x, dy = kSeenFirst ? b.y - a.y : a.y - b.y,
+                dz = kSeenFirst ? b.z - a.z : a.z - b.z;
+    return (int)!(fabsf(dx) > r.x) & (int)!(fabsf(dy) > r.y) & (int)!(fabsf(dz) > r.z);
+}
+
+}  // namespace see_detail
+
+// See pass over a row-order table with G lanes per seer (G consecutive lanes of a warp), for
+// launches whose seers alone do not fill the chip.  The lanes find the seer's row ranges
+// together, then take its candidates G at a time in the order of the row walk, test them
+// and compute the pair terms of those that count; the terms are queued in shared memory in
+// that order, and folded one after the other.  So every sum is the one the row walk
+// (see_rows_kernel) forms, bit for bit; only its terms are computed side by side.  Pair lists
+// are recorded and replayed the same way.  blockIdx.x / G is the CTA of the CTA table, the
+// rest which 128 / G of its seers.
+//
+// What bounds it: with one lane per seer a launch of 2,048 SPH particles is 64 warps, each
+// walking some 1,400 candidates one after the other (258 us for the density pass, 126 us for
+// the replaying force pass, at 2% of the issue slots); 32 lanes per seer take 19 and 16 us.
+// At 81,920 particles it is issue-bound (80% of the slots at 16 lanes), which is why terms
+// that cost something are computed for gathered candidates (17% of those walked pass the
+// density pass's test) and why the box test has no branches.  Folding costs every lane of a
+// seer the same few instructions per neighbour, so more lanes than the chip needs lose (the
+// sizes are at seer_lanes, runtime.cu).
+template <class P, int G, bool kWrite = false>
+__global__ void __launch_bounds__(kSeeThreads, 8) see_group_kernel(SeeLaunch L) {
+    using namespace see_detail;
+    using Term = typename P::Term;
+    constexpr uint32_t kSeers = kSeeThreads / G;
+    constexpr uint32_t kRows = G > 16 ? G : 16;  // row ranges found together
+    constexpr uint32_t kPer = kRows / G;         // of them per lane
+    constexpr int U = 2;                         // chunks in flight
+    constexpr int kList = ListOf<P>::value;
+    constexpr bool kBox = BoxOf<P>::value;
+    constexpr bool kCheap = CheapOf<P>::value;
+    constexpr uint32_t kSlots = group_slots(G);
+    // cheap terms wait here until a seer's slots are full; others pass G at a time, and the
+    // candidates that passed wait
+    // (rows of a stride that keeps 16-byte loads aligned and the groups on other banks)
+    constexpr uint32_t kPad = sizeof(Term) >= 16 ? 1 : 16 / sizeof(Term);
+    __shared__ __align__(16) Term s_terms[kSeers][(kCheap ? kSlots : G) + kPad];
+    __shared__ uint32_t s_wait[kSeers][kCheap ? 1 : kSlots + 1];
+    __shared__ uint2 s_rows[kSeers][kRows];
+
+    const uint2 cta = L.cta_table[L.cta_offset + blockIdx.x / G];
+    const uint32_t seg = cta.x;
+    const SegmentSpec S = L.specs[seg];
+    const uint32_t seg_end = S.begin + S.count;
+    const uint32_t first = cta.y + (blockIdx.x % G) * kSeers;
+    if (first >= seg_end) return;
+    const SegmentSpec T = L.specs[L.cross ? L.seen_seg : seg];
+    const BoxAcc B = L.box[L.cross ? L.seen_seg : seg];
+    const SegGrid &SG = L.grids[L.cross ? L.seen_seg : seg];
+    const Grid g = SG.g;
+    const float4 r4 = L.radii[seg];
+    // (a copy: what the walk reads of it stays in registers across its barriers)
+    const typename P::SeeCtx sctx = *reinterpret_cast<const typename P::SeeCtx *>(L.ctx + (size_t)seg * L.ctx_stride);
+    const typename P::ActCtx &actx =
+        *reinterpret_cast<const typename P::ActCtx *>(L.act_ctx + (size_t)seg * L.act_ctx_stride);
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t grp = threadIdx.x / G, sub = threadIdx.x % G;
+    const Group<G> gr(lane);
+    const uint32_t i = first + grp;
+    const bool active = i < seg_end;
+
+    float4 sp = make_float4(0.f, 0.f, 0.f, 0.f), smax = sp;
+    typename P::Seer s;
+    int lo[3] = {0, 0, 0}, hi[3] = {-1, -1, -1};
+    if (active) {
+        sp = L.io.in_f4[0][i];
+        if (kBox) smax = L.io.in_f4[1][i];
+        P::load(s, L.io, i, sctx, actx);
+        seer_cells<kBox>(sp, smax, r4, B, g, SG.pad, lo, hi);
+    }
+    const uint4 *hdr = reinterpret_cast<const uint4 *>(L.table + T.table_base);
+    const uint32_t *words = reinterpret_cast<const uint32_t *>(L.table + T.table_base) + row_entry_word(T);
+    const uint32_t dx0 = (uint32_t)g.dims[0], dy0 = (uint32_t)g.dims[1];
+    GlobalSeen<P::kSeenF4> acc;
+#pragma unroll
+    for (int k = 0; k < P::kSeenF4; ++k) acc.s[k] = L.io.in_f4[P::seen_stream(k)];
+    const float4 *pos = L.io.in_f4[0];
+    const uint32_t self = (active && L.skip_self) ? i : 0xFFFFFFFFu;
+    uint32_t pairs = 0, tested = 0;
+    Term *terms = &s_terms[grp][0];
+    uint32_t *wait = &s_wait[grp][0];
+    uint32_t head = 0, queued = 0;  // of the waiting terms or candidates (the same in a seer's lanes)
+
+    bool replayed = false;
+    if constexpr (kList == 2 && !kBox) {
+        if (L.plist.mode == 2u) {
+            const float4 rr = L.plist.rec_radii[seg];
+            const auto &rctx =
+                *reinterpret_cast<const typename P::SeeCtx *>(L.plist.rec_ctx + (size_t)seg * L.ctx_stride);
+            const bool covers = rr.x == r4.x && rr.y == r4.y && rr.z == r4.z && P::replay_ok(sctx, rctx);
+            const uint2 c = active ? L.plist.count[i] : make_uint2(0u, 0u);
+            replayed = __all_sync(0xffffffffu, covers && c.x <= L.plist.cap);
+            // counted per 32 seers, by the warp that holds the first of them
+            if (replayed && L.telemetry && lane == 0 && ((i - cta.y) & 31u) == 0) atomicAdd(L.telemetry + 5, 1ull);
+            if (replayed) {
+                const uint32_t *e = reinterpret_cast<const uint32_t *>(L.plist.idx + i);
+                const size_t stride = L.plist.stride * (size_t)4u;
+                // the next chunk's entries are loaded while this one's terms are computed
+                uint32_t j = sub < c.x ? __ldg(e + (size_t)(sub >> 2) * stride + (sub & 3u)) : self;
+                for (uint32_t t = sub; __any_sync(0xffffffffu, t - sub < c.x); t += G) {
+                    const uint32_t f = t + G;
+                    const uint32_t next = f < c.x ? __ldg(e + (size_t)(f >> 2) * stride + (f & 3u)) : self;
+                    eval_terms<P, G>(s, sp, t < c.x && j != self, j, pos, acc, terms, gr, sctx);
+                    j = next;
+                }
+                if (sub == 0 && active) pairs += c.y + ((!L.skip_self && box_hit(sp, sp, r4)) ? 1u : 0u);
+            }
+        }
+    }
+    if (L.telemetry && threadIdx.x == 0 && blockIdx.x % G == 0) atomicAdd(L.telemetry + 2, 1ull);
+
+    if (!replayed) {
+        const bool recording = kList == 1 && !kBox && L.plist.mode == 1u;
+        const uint32_t ny = (uint32_t)(hi[1] - lo[1] + 1);
+        const uint32_t nrows = active ? ny * (uint32_t)(hi[2] - lo[2] + 1) : 0u;
+        if (L.telemetry && lane == 0) atomicAdd(L.telemetry + 4, 1ull);
+        uint32_t listed = 0;
+        for (uint32_t rb = 0; __any_sync(0xffffffffu, rb < nrows); rb += kRows) {
+            // the next kRows rows' ranges, as {end in the flat order, first agent - begin in it}
+            uint32_t len[kPer], j0[kPer], sum = 0;
+#pragma unroll
+            for (uint32_t k = 0; k < kPer; ++k) {
+                const uint32_t r = rb + sub * kPer + k;
+                uint2 jr = make_uint2(0u, 0u);
+                if (r < nrows)
+                    jr = row_range(words, hdr, ((uint32_t)lo[2] + r / ny) * dy0 + (uint32_t)lo[1] + r % ny, dx0, lo[0],
+                                   hi[0]);
+                j0[k] = jr.x;
+                len[k] = jr.y > jr.x ? jr.y - jr.x : 0u;
+                sum += len[k];
+            }
+            uint32_t incl = sum;
+#pragma unroll
+            for (int o = 1; o < G; o <<= 1) {
+                const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o, G);
+                if (sub >= (uint32_t)o) incl += v;
+            }
+            const uint32_t total = __shfl_sync(0xffffffffu, incl, G - 1, G);
+            uint32_t at = incl - sum;
+#pragma unroll
+            for (uint32_t k = 0; k < kPer; ++k) {
+                s_rows[grp][sub * kPer + k] = make_uint2(at + len[k], j0[k] - at);
+                at += len[k];
+            }
+            __syncwarp();
+            // this lane's candidates are the flat indices sub, sub + G, ...
+            uint32_t row = 0;
+            uint2 cur = s_rows[grp][0];
+            const uint32_t most = __reduce_max_sync(0xffffffffu, total);
+            for (uint32_t f = sub; f - sub < most; f += U * G) {
+                uint32_t j[U], v[U];
+                float4 b[U], bm[U];
+                bool kept[U];
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    const uint32_t at_u = f + u * G;
+                    j[u] = self;
+                    b[u] = sp;
+                    if (at_u < total) {
+                        while (at_u >= cur.x) cur = s_rows[grp][++row];
+                        j[u] = at_u + cur.y;
+                        b[u] = __ldg(pos + j[u]);
+                        if (kBox) bm[u] = __ldg(L.io.in_f4[1] + j[u]);
+                        ++tested;
+                    }
+                }
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    const bool valid = f + u * G < total;
+                    bool hit;
+                    if constexpr (kBox)
+                        hit = valid && j[u] != self && boxes_hit(sp, smax, b[u], bm[u], r4);
+                    else
+                        hit = (int)valid & (int)box_hit_flat<P>(sp, b[u], r4);
+                    if constexpr (GateOf<P>::value && !kBox) {
+                        // as the gated row walk: the seer's own pass is counted here and
+                        // comes off the counter below
+                        pairs += hit ? 1u : 0u;
+                        kept[u] = (int)hit & (int)(SelfSafeOf<P>::value || j[u] != self) & (int)P::keep(sp, b[u], sctx);
+                    } else {
+                        kept[u] = (int)hit & (int)(j[u] != self);
+                        pairs += kept[u] ? 1u : 0u;
+                    }
+                    v[u] = gr.votes(kept[u]);
+                }
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    const uint32_t rank = __popc(v[u] & gr.below);
+                    if constexpr (kList == 1 && !kBox) {
+                        if (recording) {
+                            const uint32_t slot = listed + rank;
+                            if (kept[u] && slot < L.plist.cap)
+                                reinterpret_cast<uint32_t *>(
+                                    L.plist.idx)[((size_t)(slot >> 2) * L.plist.stride + i) * 4u + (slot & 3u)] = j[u];
+                            listed += __popc(v[u]);
+                        }
+                    }
+                    if constexpr (kCheap) {
+                        if (kept[u]) P::term(s, sp, b[u], acc, j[u], sctx, terms[queued + rank]);
+                    } else {
+                        if (kept[u]) wait[(head + queued + rank) & (kSlots - 1u)] = j[u];
+                    }
+                    queued += __popc(v[u]);
+                }
+                if (__any_sync(0xffffffffu, queued > kSlots - U * G)) {
+                    if constexpr (kCheap) {
+                        fold_terms<P, kSlots>(s, terms, queued, sctx);
+                        queued = 0;
+                    } else {
+                        __syncwarp();
+                        do {
+                            const uint32_t m = min(queued, (uint32_t)G);
+                            eval_terms<P, G>(s, sp, sub < m, wait[(head + sub) & (kSlots - 1u)], pos, acc, terms, gr,
+                                             sctx);
+                            head += m;
+                            queued -= m;
+                        } while (__any_sync(0xffffffffu, queued > kSlots - U * G));
+                    }
+                }
+            }
+            __syncwarp();  // the ranges are read before the next ones are written
+        }
+        if constexpr (GateOf<P>::value && !kBox) {
+            const uint32_t own = active && box_hit(sp, sp, r4) ? 1u : 0u;
+            if constexpr (kList == 1) {
+                if (recording) {
+                    uint32_t all = pairs;
+#pragma unroll
+                    for (int o = 1; o < G; o <<= 1) all += __shfl_xor_sync(0xffffffffu, all, o);
+                    if (active && sub == 0) L.plist.count[i] = make_uint2(listed, all - own);
+                }
+            }
+            if (sub == 0 && L.skip_self) pairs -= own;
+        }
+    }
+    if constexpr (kCheap) {
+        fold_terms<P, kSlots>(s, terms, queued, sctx);
+    } else {
+        __syncwarp();
+        while (__any_sync(0xffffffffu, queued > 0u)) {
+            const uint32_t m = min(queued, (uint32_t)G);
+            eval_terms<P, G>(s, sp, sub < m, wait[(head + sub) & (kSlots - 1u)], pos, acc, terms, gr, sctx);
+            head += m;
+            queued -= m;
+        }
+    }
+    if (active && sub == 0) P::finish(s, sp, L.io, i, sctx, actx);
+    if (L.pairs) {
+        uint32_t w = warp_sum_u(pairs);
+        if (lane == 0 && w) atomicAdd(L.pairs, (unsigned long long)w);
+    }
+    if (L.telemetry) {
+        uint32_t w = warp_sum_u(tested);
+        if (lane == 0 && w) atomicAdd(L.telemetry, (unsigned long long)w);
+    }
+    if constexpr (kWrite) {
+        using C = typename CodecOf<P>::type;
+        __shared__ __align__(16) uint32_t wt_sm[kSeers * (C::kAgentBytes / 4)];
+        uint32_t *wt = L.wt[seg];
+        if (wt) {
+            __syncthreads();  // the records written by each seer's first lane
+            write_through_cta<C, kSeers>(L, wt, first, S.begin, seg_end, wt_sm);
+        }
     }
 }
 

@@ -95,6 +95,7 @@ struct SeeLaunch {
     uint32_t *const *wt;
     uint32_t wt_program;
     PairList plist;
+    uint32_t lanes;  // row order: lanes per seer (1, 8, 16 or 32; see_group_kernel above 1)
 };
 
 struct ActLaunch {

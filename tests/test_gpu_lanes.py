@@ -1,0 +1,78 @@
+"""GPU: see passes whose seers share several lanes (small and middle launches) give the bits
+of the row walk with one lane per seer.  The terms of a seer's neighbours are the same
+floats, folded in the same order, so records and pair counts must be equal byte for byte
+(no tolerance).  The hit-mask tuning keeps one lane per seer, walks in the same order and
+keeps no pair lists, so it is the comparison for every model."""
+import numpy as np
+import pytest
+
+from tay_gb300 import api
+from tay_gb300 import models as M
+from tay_gb300 import workloads as W
+
+pytestmark = pytest.mark.gpu
+
+
+def _records(model, n):
+    if model == "test":
+        ps = W.basic_points(n, seed=91, side=1000.0 * (n / 1e5) ** (1 / 3) + 1.0)
+        return M.test_setup(), M.records(M.TEST_RECORD, ps.p, ps.v)
+    if model == "box":
+        b = W.box_agents(n, seed=92)
+        return M.box_setup(), M.box_records(b.lo, b.hi, b.v)
+    if model == "boids":  # 64 neighbours inside the box, both halves of the separation test
+        ps = W.basic_points(n, seed=93, side=(125.0 * n) ** (1 / 3))
+        return M.boids_setup(r=10.0, part=10.0), M.records(M.BOIDS_RECORD, ps.p, ps.v)
+    if model == "heap":  # every particle inside every other's support: the pair lists overflow
+        p = np.full((n, 4), 0.05, np.float32)
+        p[:, :3] += np.random.default_rng(94).uniform(0, 0.01, (n, 3)).astype(np.float32)
+        p[:, 3] = 0.0
+        return M.sph_setup(mb=64), M.records(M.SPH_RECORD, p, np.zeros((n, 4), np.float32))
+    side = int(np.ceil(n ** (1 / 3)))
+    sph = W.sph_dam(side, side, side)
+    return M.sph_setup(mb=64), M.records(M.SPH_RECORD, sph.points.p[:n], sph.points.v[:n])
+
+
+def _run(setup, recs, steps, **tuning):
+    api.set_tuning(**tuning)
+    try:
+        b = api.Batch([(setup, recs)])
+        try:
+            b.push()
+            pairs = [b.run(1)[1] for _ in range(steps)]
+            return M.by_id(b.fetch(0)).tobytes(), pairs
+        finally:
+            b.close()
+    finally:
+        api.set_tuning()
+
+
+# a single agent, part of a CTA, a CTA and one more, and sizes at 32, 16, 8 and 1 lanes per
+# seer for each model's density
+@pytest.mark.parametrize("model,n", [
+    ("test", 1), ("test", 2), ("test", 127), ("test", 129), ("test", 2500), ("test", 4097), ("test", 12289),
+    ("test", 40000), ("test", 60001), ("box", 3), ("box", 3001), ("box", 12289), ("boids", 33), ("boids", 2049),
+    ("boids", 8193), ("boids", 30001), ("sph", 5), ("sph", 4097), ("sph", 20001), ("sph", 40001), ("sph", 130000),
+    ("heap", 700)])
+def test_shared_lanes_equal_one_lane(gpu, model, n):
+    setup, recs = _records(model, n)
+    assert _run(setup, recs, 3) == _run(setup, recs, 3, hit_masks=1)
+
+
+def test_two_groups_read_every_step(gpu):
+    """Groups of a state that see each other, each launch over one group's seers, and the
+    records written through after every run."""
+    a, b = W.basic_points(3001, seed=95, side=310.0), W.basic_points(1999, seed=96, side=310.0)
+    recs = [M.records(M.TEST_RECORD, x.p, x.v) for x in (a, b)]
+    passes = [("see", 0, 0, False), ("see", 0, 1, False), ("see", 1, 0, False), ("act", 0), ("act", 1)]
+    see, act = M.test_contexts()
+    out = []
+    for tuning in ({}, {"hit_masks": 1}):
+        api.set_tuning(**tuning)
+        try:
+            out.append(M.run_groups(M.TEST_RECORD, ("agent_see", "agent_act"), recs, passes, see, act, 50.0, 50.0, 4,
+                                    host_loop="read" if not tuning else None))
+        finally:
+            api.set_tuning()
+    for x, y in zip(*out):
+        assert x.tobytes() == y.tobytes()
