@@ -155,7 +155,6 @@ extern "C" int tgpu_see_noalloc(const float *positions, unsigned n, const float 
     spec.fixed_box = 0;
     for (int a = 0; a < 3; ++a) {
         spec.part[a] = min_part_sizes[a] > 0.0f ? min_part_sizes[a] : 1.0f;
-        spec.reach[a] = radii[a];
     }
     const float4 r4 = make_float4(radii[0], radii[1], radii[2], radii[3]);
     noalloc_setup_kernel<<<152, 256, 0, st>>>(scratch, spec, r4, n);

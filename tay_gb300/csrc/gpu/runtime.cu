@@ -9,7 +9,6 @@
 #include <dlfcn.h>
 
 #include <algorithm>
-#include <array>
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
@@ -106,6 +105,11 @@ uint32_t next_pow2(uint32_t v) {
     while (p < v) p <<= 1;
     return p;
 }
+
+// Agents per cell that programs with a recording pass aim at, and the agents of a batch from
+// which they do (fill_multiple).
+constexpr float kFill = 32.0f / 27.0f;
+constexpr uint32_t kFillAgents = 16384;
 
 uint32_t log2u(uint32_t v) {
     uint32_t n = 0;
@@ -317,12 +321,17 @@ int tgpu::prepare_specs(TgpuBatch *b) {
     for (int s = 0; s < b->nseg; ++s) {
         SegmentSpec &sp = next[s];
         const HostSeg &h = b->hs[s];
+        sp.fill = b->fill;
         uint32_t want[3] = {2, 2, 2};
+        float exts[3];
+        for (int a = 0; a < 3; ++a)
+            exts[a] = std::max(0.0f, h.g.box_fixed ? h.g.box_max[a] - h.g.box_min[a] : h.host_max[a] - h.host_min[a]);
+        const double multiple = fill_multiple((float)sp.count, exts, sp.part, seg_dims(sp), sp.fill);
         for (int a = 0; a < seg_dims(sp); ++a) {
             float lo = h.g.box_fixed ? h.g.box_min[a] : h.host_min[a];
             float hi = h.g.box_fixed ? h.g.box_max[a] : h.host_max[a];
             float ext = hi > lo ? hi - lo : 0.0f;
-            double cells = floor((double)ext / (double)sp.part[a]) + 1.0;
+            double cells = floor((double)ext / ((double)sp.part[a] * multiple)) + 1.0;
             want[a] = std::min(1024u, next_pow2((uint32_t)std::min(1024.0, std::max(2.0, ceil(cells * 1.1)))));
         }
         // Morton order: one bound for all axes; row order: each axis its own bound, so
@@ -348,21 +357,34 @@ int tgpu::prepare_specs(TgpuBatch *b) {
         table_total += cap;
         max_key_bits = std::max(max_key_bits, seg_key_bits);
     }
+    // tables of smaller cells that cannot be had: the part size's
+    auto coarser = [b]() {
+        b->fill = 0.0f;
+        b->specs_dirty = true;
+        return prepare_specs(b);
+    };
+    if (table_total > 0xFFFFFFFFull && b->fill > 0.0f) return coarser();
     if (table_total > 0xFFFFFFFFull)
         return fail(TGPU_ERR_ARG, "cell tables too large (%llu entries)", (unsigned long long)table_total);
     const uint32_t key_bits = max_key_bits;
     const bool same = b->table && key_bits == b->key_bits &&
                       !memcmp(next.data(), b->specs.data(), sizeof(SegmentSpec) * b->nseg);
     if (same) return TGPU_OK;  // the table is left clean by every completed step
-    b->specs = next;
-    b->key_bits = key_bits;
     if (table_total > b->table_entries) {
         cudaFree(b->table);
         b->table = nullptr;
         b->table_entries = 0;
-        CK(cudaMalloc(&b->table, table_total * sizeof(uint2)));
+        const cudaError_t e = cudaMalloc(&b->table, table_total * sizeof(uint2));
+        if (e == cudaErrorMemoryAllocation && b->fill > 0.0f) {
+            cudaGetLastError();
+            b->table = nullptr;
+            return coarser();
+        }
+        CK(e);
         b->table_entries = table_total;
     }
+    b->specs = next;
+    b->key_bits = key_bits;
     CK(cudaMemsetAsync(b->table, 0, b->table_entries * sizeof(uint2), b->st));
     CK(cudaMemcpyAsync(b->d_specs, b->specs.data(), sizeof(SegmentSpec) * b->nseg, cudaMemcpyHostToDevice, b->st));
     for (auto &kv : b->graphs) cudaGraphExecDestroy(kv.second);
@@ -849,8 +871,7 @@ void tgpu_batch_destroy(TgpuBatch *b) { free_batch(b); }
 namespace {
 
 // Segments of a new batch, one per group: packed agent ranges, radix tiles and see CTAs.
-// reach[g][a] is the largest see radius per axis of the passes whose seers are group g.
-int add_segments(TgpuBatch *b, const TgpuGroup *groups, int group_count, const std::vector<std::array<float, 3>> &reach) {
+int add_segments(TgpuBatch *b, const TgpuGroup *groups, int group_count) {
     uint32_t total = 0;
     for (int s = 0; s < group_count; ++s) {
         const TgpuGroup &g = groups[s];
@@ -879,7 +900,6 @@ int add_segments(TgpuBatch *b, const TgpuGroup *groups, int group_count, const s
             if (a == 0 && b->cell_order == kOrderRows) sp.part[a] *= g_tuning.x_cell_factor;
             sp.box_min[a] = g.box_min[a];
             sp.box_max[a] = g.box_max[a];
-            sp.reach[a] = reach[s][a];
         }
         sp.tile_begin = (uint32_t)b->tile_seg.size();
         sp.tile_count = (g.count + kSortTile - 1) / kSortTile;
@@ -1082,15 +1102,9 @@ int tgpu_batch_create(const TgpuGroup *groups, int group_count, TgpuBatch **out)
                         g0.passes[k].func_name ? g0.passes[k].func_name : "(null)", m->name);
     const int program = match_program(m, g0);
     if (program < 0) return fail(TGPU_ERR_PROGRAM, "pass sequence not supported by device model '%s'", m->name);
-    std::vector<std::array<float, 3>> reach(group_count);
     for (int s = 0; s < group_count; ++s) {
         const TgpuGroup &g = groups[s];
         if (!g.passes || match_program(m, g) != program) return fail(TGPU_ERR_ARG, "group %d: pass sequence differs from group 0", s);
-        for (int a = 0; a < 3; ++a) {
-            reach[s][a] = 0.0f;
-            for (int k = 0; k < g.pass_count; ++k)
-                if (g.passes[k].is_see) reach[s][a] = std::max(reach[s][a], g.passes[k].radii[a]);
-        }
     }
 
     TgpuBatch *b = new TgpuBatch();
@@ -1100,9 +1114,18 @@ int tgpu_batch_create(const TgpuGroup *groups, int group_count, TgpuBatch **out)
     b->use_graphs = g_tuning.use_graphs != 0;
     b->cell_order = g_tuning.cell_order == kOrderRows ? kOrderRows : kOrderMorton;
     b->hit_masks = g_tuning.hit_masks ? 1u : 0u;
-    int rc = add_segments(b, groups, group_count, reach);
+    int rc = add_segments(b, groups, group_count);
     if (!rc) rc = alloc_batch(b);
     const ProgramDesc &pd = m->programs[program];
+    // Cells below the part size for programs with a pass that records its neighbours (the walk
+    // is most of their step), unless a tuning says which cells to use; a property of the
+    // program, not of whether lists are kept, so that lists never change a result.
+    const TgpuTuning standard = default_tuning();
+    const bool own_cells =
+        g_tuning.cell_multiple != standard.cell_multiple || g_tuning.x_cell_factor != standard.x_cell_factor;
+    bool records = false;
+    for (int k = 0; k < pd.kernels; ++k) records = records || m->kernels[pd.kernel_index[k]].pair_list == 1;
+    if (records && !own_cells && b->cell_order == kOrderRows && b->total > kFillAgents) b->fill = kFill;
     int cursor = 0;
     for (int k = 0; k < pd.kernels && !rc; ++k) {
         KernelRun r{};
@@ -1133,8 +1156,6 @@ int tgpu_state_create(const TgpuGroup *groups, int group_count, const TgpuStateP
     *out = nullptr;
     const ModelDesc *m = find_model(passes[0].pass.func_name ? passes[0].pass.func_name : "");
     if (!m) return fail(TGPU_ERR_UNKNOWN_FUNC, "no device model provides '%s'", passes[0].pass.func_name);
-    std::vector<std::array<float, 3>> reach(group_count);
-    for (auto &r : reach) r = {0.0f, 0.0f, 0.0f};
     std::vector<int> see_passes(group_count, 0);
     std::vector<const KernelDesc *> kernels(pass_count);
     for (int k = 0; k < pass_count; ++k) {
@@ -1156,7 +1177,6 @@ int tgpu_state_create(const TgpuGroup *groups, int group_count, const TgpuStateP
             if (++see_passes[sp.seer_group] > 1 && !d.accumulates)
                 return fail(TGPU_ERR_PROGRAM, "group %d: several '%s' see passes, and the see function of model '%s' does not accumulate",
                             sp.seer_group, fn, m->name);
-            for (int a = 0; a < 3; ++a) reach[sp.seer_group][a] = std::max(reach[sp.seer_group][a], sp.pass.radii[a]);
         }
     }
 
@@ -1168,7 +1188,7 @@ int tgpu_state_create(const TgpuGroup *groups, int group_count, const TgpuStateP
     b->cell_order = g_tuning.cell_order == kOrderRows ? kOrderRows : kOrderMorton;
     b->hit_masks = g_tuning.hit_masks ? 1u : 0u;
     b->state_passes.assign(passes, passes + pass_count);
-    int rc = add_segments(b, groups, group_count, reach);
+    int rc = add_segments(b, groups, group_count);
     if (!rc) rc = alloc_batch(b);
     for (int k = 0; k < pass_count && !rc; ++k) {
         const TgpuStatePass &sp = passes[k];

@@ -69,6 +69,7 @@ struct TgpuBatch {
     std::vector<TgpuStatePass> state_passes;   // tgpu_state_create: the state's pass list
     uint32_t tiles = 0, ctas = 0, key_bits = 0;
     bool specs_dirty = true;
+    float fill = 0.0f;  // SegmentSpec::fill of every segment
 
     SegmentSpec *d_specs = nullptr;
     uint32_t *d_tile_seg = nullptr;
