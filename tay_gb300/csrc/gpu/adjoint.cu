@@ -190,9 +190,13 @@ void recorded_step(TgpuAdjoint *a, Record *r, const StepList *pl = nullptr) {
     TgpuBatch *b = a->b;
     cudaStream_t st = b->st;
     SortLaunch L = sort_launch(b);
-    launch_box(L, st);
     uint32_t *skeys = nullptr, *perm = nullptr;
-    launch_sort(L, st, &skeys, &perm);
+    if (L.cluster_blocks) {
+        launch_cluster_sort(L, st, &skeys, &perm);
+    } else {
+        launch_box(L, st);
+        launch_sort(L, st, &skeys, &perm);
+    }
     GatherSet g{};
     for (int c = 0; c < b->m->nf4; ++c) {
         if (b->m->role_f4[c] != kState) continue;

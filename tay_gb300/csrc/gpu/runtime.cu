@@ -390,11 +390,12 @@ int tgpu::prepare_specs(TgpuBatch *b) {
     for (auto &kv : b->graphs) cudaGraphExecDestroy(kv.second);
     b->graphs.clear();
     // box reset, bounding box (+ grids), keys and histograms (+ digit offsets), one kernel
-    // per radix pass, cell table (+ reorder), the passes, and the table clear when it is
+    // per radix pass (or one kernel for all of these), cell table (+ reorder), the passes, and the table clear when it is
     // a kernel (Morton order, or more segments than separate header memsets)
     const int passes = sort_passes(b->key_bits);
     const bool clear_kernel = b->cell_order != kOrderRows || b->nseg > kMemsetClearSegments;
-    b->launches_per_step = 2 + 1 + passes + 1 + (int)b->runs.size() + (clear_kernel ? 1 : 0);
+    const int sort = b->cluster_blocks ? 1 : 2 + 1 + passes;
+    b->launches_per_step = sort + 1 + (int)b->runs.size() + (clear_kernel ? 1 : 0);
     return TGPU_OK;
 }
 
@@ -439,6 +440,7 @@ SortLaunch tgpu::sort_launch(TgpuBatch *b) {
     L.segments = (uint32_t)b->nseg;
     L.tiles = b->tiles;
     L.key_bits = b->key_bits;
+    L.cluster_blocks = b->cluster_blocks;
     return L;
 }
 
@@ -495,11 +497,14 @@ void tgpu::enqueue_step(TgpuBatch *b, const StepEvents *E, bool write_through) {
     cudaStream_t st = b->st;
     SortLaunch L = sort_launch(b);
     mark(E, 0, st);
-    launch_box(L, st);
+    if (!L.cluster_blocks) launch_box(L, st);
     mark(E, 1, st);
     uint32_t *skeys = nullptr, *perm = nullptr;
     mark(E, 2, st);
-    launch_sort(L, st, &skeys, &perm);
+    if (L.cluster_blocks)
+        launch_cluster_sort(L, st, &skeys, &perm);
+    else
+        launch_sort(L, st, &skeys, &perm);
     mark(E, 3, st);
     GatherSet g{};
     for (int c = 0; c < b->m->nf4; ++c) {
@@ -966,6 +971,9 @@ int alloc_batch(TgpuBatch *b) {
     b->d_err = reinterpret_cast<uint32_t *>(b->d_status + 9);
     CKR(cudaMalloc(&b->d_aos, (size_t)m->agent_bytes * n));
     b->ctx_stride = (std::max(m->see_ctx_bytes, m->act_ctx_bytes) + 15u) & ~15u;
+    uint32_t largest = 0;
+    for (const auto &sp : b->specs) largest = std::max(largest, sp.count);
+    b->cluster_blocks = cluster_sort_blocks((uint32_t)b->nseg, largest);
     return TGPU_OK;
 }
 

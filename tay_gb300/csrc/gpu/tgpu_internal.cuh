@@ -53,8 +53,7 @@ struct SegmentSpec {
     float box_max[3];
 };
 
-// Per-step grid, derived on the device from the bounding box.  Every kernel derives
-// it with the same function from the same inputs, so all kernels agree bit for bit.
+// Per-step grid, derived on the device from the bounding box (derive_grid).
 struct Grid {
     float origin[3];
     float inv_cs[3];
@@ -161,49 +160,6 @@ TGPU_HD float fill_multiple(float count, const float *ext, const float *part, in
     return m > 0.7f || !(m > 0.0f) ? 1.0f : (m < 0.25f ? 0.25f : m);
 }
 
-TGPU_HD Grid derive_grid(const SegmentSpec &s, const float *mn, const float *mx) {
-    Grid g;
-    float cs[3], ext[3];
-    int d[3];
-    for (int i = 0; i < 3; ++i) {
-        ext[i] = mx[i] - mn[i];
-        if (!(ext[i] >= 0.0f) || ext[i] > 3.0e38f) ext[i] = 0.0f;
-        cs[i] = s.part[i] > 0.0f ? s.part[i] : 1.0f;
-    }
-    const float multiple = fill_multiple((float)s.count, ext, cs, seg_dims(s), s.fill);
-    for (int i = 0; i < 3; ++i) {
-        cs[i] *= multiple;
-        float cells = floorf(ext[i] / cs[i]) + 1.0f;
-        if (cells > (float)axis_max(s, i)) cs[i] = ext[i] / ((float)axis_max(s, i) - 0.5f);
-        d[i] = clamp_cells(floorf(ext[i] / cs[i]) + 1.0f, axis_max(s, i));
-        if (i >= seg_dims(s)) {
-            // an axis the space does not have: one cell spanning it
-            d[i] = 1;
-            cs[i] = ext[i] > cs[i] ? ext[i] : cs[i];
-        }
-    }
-    for (int iter = 0; iter < 64; ++iter) {
-        if (table_fits(s, d)) break;
-        for (int i = 0; i < seg_dims(s); ++i) {
-            cs[i] *= 1.25f;
-            d[i] = clamp_cells(floorf(ext[i] / cs[i]) + 1.0f, axis_max(s, i));
-        }
-    }
-    if (!table_fits(s, d)) {
-        for (int i = 0; i < 3; ++i) {
-            d[i] = 1;
-            cs[i] = ext[i] > cs[i] ? ext[i] : cs[i];
-        }
-    }
-    for (int i = 0; i < 3; ++i) {
-        g.origin[i] = mn[i];
-        g.cs[i] = cs[i];
-        g.inv_cs[i] = 1.0f / cs[i];
-        g.dims[i] = d[i];
-    }
-    return g;
-}
-
 TGPU_HD int cell_coord(float p, float origin, float inv_cs, int dim) {
     int c = (int)floorf((p - origin) * inv_cs);
     return c < 0 ? 0 : (c >= dim ? dim - 1 : c);
@@ -296,38 +252,88 @@ TGPU_HD uint32_t cell_key(const SegmentSpec &s, uint32_t x, uint32_t y, uint32_t
     return morton3(x, y, z);
 }
 
-// The step's grid of a segment: from its fixed box, or from the bounding box of its
-// positions accumulated by the box kernel.
-TGPU_HD Grid segment_grid(const SegmentSpec &s, const BoxAcc &b) {
-    float mn[3], mx[3];
-    for (int i = 0; i < 3; ++i) {
-        mn[i] = s.fixed_box ? s.box_min[i] : ordered_to_float(b.lo[i]);
-        mx[i] = s.fixed_box ? s.box_max[i] : ordered_to_float(b.hi[i]);
-    }
-    return derive_grid(s, mn, mx);
-}
-
-// Largest rounding error, in cells, of a cell coordinate computed as
+// A segment's grid for one step with its rounding pad, derived once per step from the
+// bounding box (derive_grid) and read by every later kernel of the step.  The pad is the
+// largest rounding error, in cells, of a cell coordinate computed as
 // floor((p - origin) * inv_cs): a few ulps of the largest coordinate magnitude plus the
 // relative error of the multiply on coordinates up to 1024 cells.
-TGPU_D float grid_pad(const Grid &g, const SegmentSpec &s, const BoxAcc &b) {
-    float m = 0.0f, csmin = g.cs[0];
-    for (int a = 0; a < 3; ++a) {
-        float lo = s.fixed_box ? s.box_min[a] : ordered_to_float(b.lo[a]);
-        float hi = s.fixed_box ? s.box_max[a] : ordered_to_float(b.hi[a]);
-        m = fmaxf(m, fmaxf(fabsf(lo), fabsf(hi)));
-        csmin = fminf(csmin, g.cs[a]);
-    }
-    float ulp = m * 1.1920929e-7f;  // 2^-23
-    return fmaxf(1.0f / 512.0f, 16.0f * ulp / csmin + 1024.0f * 4.0f * 1.1920929e-7f);
-}
-
-// A segment's grid for one step with its rounding pad (grid_pad), derived once per step
-// from the bounding box by the grid kernel and read by every later kernel of the step.
 struct SegGrid {
     Grid g;
     float pad;
 };
+
+#ifdef __CUDACC__
+// Derives a segment's grid into *out from its fixed box, or from the bounding box of its
+// positions (the ordered encodings of axis `lane` in lanes 0..2; other lanes pass anything).
+// One warp, an axis per lane: every step waits for it, and by one thread, its some ten
+// divisions one after the other, a step of 100,000 agents took 1 us longer.
+// `s` in global memory: its per-axis fields are picked by the lane.
+TGPU_D void derive_grid(const SegmentSpec &s, uint32_t box_lo, uint32_t box_hi, SegGrid *out) {
+    const uint32_t lane = threadIdx.x & 31u;
+    const int i = lane < 3u ? (int)lane : 2;
+    const float mn = s.fixed_box ? s.box_min[i] : ordered_to_float(box_lo);
+    const float mx = s.fixed_box ? s.box_max[i] : ordered_to_float(box_hi);
+    const bool axis = i < seg_dims(s);
+    const uint32_t axis_cells = axis_max(s, i);
+    const float most = (float)axis_cells;
+    float ext = mx - mn;
+    if (!(ext >= 0.0f) || ext > 3.0e38f) ext = 0.0f;
+    float cs = s.part[i] > 0.0f ? s.part[i] : 1.0f;
+    if (s.fill > 0.0f) {
+        float exts[3], parts[3];
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            exts[a] = __shfl_sync(0xffffffffu, ext, a);
+            parts[a] = __shfl_sync(0xffffffffu, cs, a);
+        }
+        cs *= fill_multiple((float)s.count, exts, parts, seg_dims(s), s.fill);
+    }
+    float cells = floorf(ext / cs) + 1.0f;
+    if (cells > most) {
+        cs = ext / (most - 0.5f);
+        cells = floorf(ext / cs) + 1.0f;
+    }
+    int d = clamp_cells(cells, axis_cells);
+    if (!axis) {
+        // an axis the space does not have: one cell spanning it
+        d = 1;
+        cs = ext > cs ? ext : cs;
+    }
+    int dims[3];
+    bool fits = false;
+    for (int iter = 0; iter < 65; ++iter) {
+#pragma unroll
+        for (int a = 0; a < 3; ++a) dims[a] = __shfl_sync(0xffffffffu, d, a);
+        fits = table_fits(s, dims);
+        if (fits || iter == 64) break;
+        if (axis) {
+            cs *= 1.25f;
+            d = clamp_cells(floorf(ext / cs) + 1.0f, axis_cells);
+        }
+    }
+    if (!fits) {
+        d = 1;
+        cs = ext > cs ? ext : cs;
+    }
+    const float m = fmaxf(fabsf(mn), fabsf(mx));
+    float all = 0.0f, csmin = __shfl_sync(0xffffffffu, cs, 0);
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        all = fmaxf(all, __shfl_sync(0xffffffffu, m, a));
+        csmin = fminf(csmin, __shfl_sync(0xffffffffu, cs, a));
+    }
+    if (lane < 3u) {
+        out->g.origin[lane] = mn;
+        out->g.cs[lane] = cs;
+        out->g.inv_cs[lane] = 1.0f / cs;
+        out->g.dims[lane] = d;
+    }
+    if (lane == 0) {
+        const float ulp = all * 1.1920929e-7f;  // 2^-23
+        out->pad = fmaxf(1.0f / 512.0f, 16.0f * ulp / csmin + 1024.0f * 4.0f * 1.1920929e-7f);
+    }
+}
+#endif
 
 // Device-side error word: kernels never trap; they record the first failure here and
 // the host turns it into TAY_ERROR_CUDA.
