@@ -89,6 +89,9 @@ struct SphAdjointKernels {
 const SphAdjointKernels *sph_adjoint_kernels();
 
 const ModelDesc *model_test_basic();
+// The test model's see pass from zero, its sums (float4 out stream 2) at the slots of u32
+// stream 0 (used by noalloc.cu).
+void launch_see_out(const SeeLaunch &L, cudaStream_t st);
 const ModelDesc *model_boids();
 const ModelDesc *model_sph();
 const ModelDesc *model_box();

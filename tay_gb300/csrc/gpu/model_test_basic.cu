@@ -105,6 +105,23 @@ struct SeeOnly : See {
     }
 };
 
+// agent_see from zero, each seer's sums to its place before the sort: out stream BBUF at
+// index u32[0] (the allocation-free pass; in its caller's order without a pass of its own).
+struct SeeOut : See {
+    using SeeCtx = test_basic::SeeCtx;
+    using ActCtx = test_basic::SeeCtx;
+    using Seer = test_basic::Seer;
+    static constexpr int kSeenF4 = 1;
+    TGPU_D static int seen_stream(int) { return POS; }
+    TGPU_D static void load(Seer &s, const PassIO &, uint32_t, const SeeCtx &, const ActCtx &) {
+        s.bx = s.by = s.bz = 0.0f;
+        s.count = 0;
+    }
+    TGPU_D static void finish(Seer &s, const float4 &, const PassIO &io, uint32_t i, const SeeCtx &, const ActCtx &) {
+        io.out_f4[BBUF][io.in_u32[0][i]] = make_float4(s.bx, s.by, s.bz, __int_as_float(s.count));
+    }
+};
+
 struct SeeAct : See {
     using SeeCtx = test_basic::SeeCtx;
     using Codec = test_basic::Codec;
@@ -196,6 +213,8 @@ const ModelDesc kModel = {
 };
 
 }  // namespace test_basic
+
+void launch_see_out(const SeeLaunch &L, cudaStream_t st) { launch_see_t<test_basic::SeeOut>(L, 0, st); }
 
 const ModelDesc *model_test_basic() { return &test_basic::kModel; }
 

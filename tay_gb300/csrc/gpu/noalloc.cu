@@ -26,8 +26,7 @@
 //     refuses to start and leaves that error in place for its owner.
 #include <cstdio>
 
-#include "model.cuh"
-#include "tay_gpu.h"
+#include "runtime_internal.cuh"
 
 namespace tgpu {
 namespace {
@@ -36,6 +35,9 @@ constexpr uint32_t kNoallocMaxAgents = 65536;
 constexpr uint32_t kNoallocAxisCells = 64;
 constexpr uint32_t kNoallocTable = kNoallocAxisCells * kNoallocAxisCells * kNoallocAxisCells;
 constexpr uint32_t kNoallocTiles = kNoallocMaxAgents / kSortTile;
+// Neighbours a seer is taken to have (those of the 100,000-agent test workload): the call
+// sees no extent before it runs.
+constexpr double kNoallocMates = 100.0;
 constexpr uint32_t kNoallocCtas = kNoallocMaxAgents / kSeeThreads;
 
 constexpr size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
@@ -57,8 +59,7 @@ constexpr size_t kOffSortScratch = align256(kOffVals1 + sizeof(uint32_t) * kNoal
 constexpr size_t kOffErr = align256(kOffSortScratch + sort_scratch_bytes(1, kNoallocTiles));
 constexpr size_t kOffTable = align256(kOffErr + sizeof(uint32_t));
 constexpr size_t kOffPos = align256(kOffTable + sizeof(uint2) * kNoallocTable);
-constexpr size_t kOffAcc = align256(kOffPos + sizeof(float4) * kNoallocMaxAgents);
-constexpr size_t kNoallocBytes = align256(kOffAcc + sizeof(float4) * kNoallocMaxAgents);
+constexpr size_t kNoallocBytes = align256(kOffPos + sizeof(float4) * kNoallocMaxAgents);
 static_assert(kNoallocBytes < (8u << 20), "scratch stays modest");
 
 }  // namespace
@@ -68,8 +69,9 @@ static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoallocBytes];
 
 namespace {
 
-// Writes the one-segment description, the tile and CTA tables, the radii and context,
-// and clears the pair counter, the accumulators and the cell table.
+// Writes the one-segment description, the tile and CTA tables, the radii and context, and
+// clears the pair counter, the error word and the headers of the cell table (its entries are
+// read only where a call writes them).
 __global__ void noalloc_setup_kernel(unsigned char *scratch, SegmentSpec spec, float4 radii, uint32_t n) {
     const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t threads = gridDim.x * blockDim.x;
@@ -78,22 +80,15 @@ __global__ void noalloc_setup_kernel(unsigned char *scratch, SegmentSpec spec, f
         *reinterpret_cast<unsigned long long *>(scratch + kOffPairs) = 0ull;
         *reinterpret_cast<float4 *>(scratch + kOffRadii) = radii;
         *reinterpret_cast<float4 *>(scratch + kOffCtx) = radii;
+        *reinterpret_cast<uint32_t *>(scratch + kOffErr) = 0u;
     }
     uint32_t *tile_seg = reinterpret_cast<uint32_t *>(scratch + kOffTileSeg);
     for (uint32_t t = tid; t < spec.tile_count; t += threads) tile_seg[t] = 0u;
     uint2 *cta = reinterpret_cast<uint2 *>(scratch + kOffCta);
     const uint32_t ctas = (n + kSeeThreads - 1) / kSeeThreads;
     for (uint32_t c = tid; c < ctas; c += threads) cta[c] = make_uint2(0u, c * kSeeThreads);
-    float4 *acc = reinterpret_cast<float4 *>(scratch + kOffAcc);
-    for (uint32_t i = tid; i < n; i += threads) acc[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-    uint2 *table = reinterpret_cast<uint2 *>(scratch + kOffTable);
-    for (uint32_t c = tid; c < kNoallocTable; c += threads) table[c] = make_uint2(0u, 0u);
-}
-
-// Results back in the caller's order: out[perm[i]] = acc[i].
-__global__ void noalloc_unpermute_kernel(const uint32_t *perm, const float4 *acc, float4 *out, uint32_t n) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) out[perm[i]] = acc[i];
+    uint4 *headers = reinterpret_cast<uint4 *>(scratch + kOffTable);
+    for (uint32_t r = tid; r < spec.row_cap; r += threads) headers[r] = make_uint4(0u, 0u, 0u, 0u);
 }
 
 thread_local char g_noalloc_err[256];
@@ -151,13 +146,15 @@ extern "C" int tgpu_see_noalloc(const float *positions, unsigned n, const float 
     spec.table_cap = kNoallocTable;
     spec.tile_begin = 0;
     spec.tile_count = (n + kSortTile - 1) / kSortTile;
-    spec.axis_cells_max = kNoallocAxisCells;
+    // rows of cells as the regular path lays them out by default: x cells of half the part
+    spec.order = kOrderRows;
+    spec.axis_cells_max = spec.axis_cells_y = spec.axis_cells_z = kNoallocAxisCells;
+    spec.row_cap = kNoallocAxisCells * kNoallocAxisCells;
     spec.fixed_box = 0;
-    for (int a = 0; a < 3; ++a) {
-        spec.part[a] = min_part_sizes[a] > 0.0f ? min_part_sizes[a] : 1.0f;
-    }
+    for (int a = 0; a < 3; ++a) spec.part[a] = min_part_sizes[a] > 0.0f ? min_part_sizes[a] : 1.0f;
+    spec.part[0] *= 0.5f;
     const float4 r4 = make_float4(radii[0], radii[1], radii[2], radii[3]);
-    noalloc_setup_kernel<<<152, 256, 0, st>>>(scratch, spec, r4, n);
+    noalloc_setup_kernel<<<16, 256, 0, st>>>(scratch, spec, r4, n);
 
     SortLaunch L{};
     L.specs = reinterpret_cast<const SegmentSpec *>(scratch + kOffSpec);
@@ -176,9 +173,16 @@ extern "C" int tgpu_see_noalloc(const float *positions, unsigned n, const float 
     L.tiles = spec.tile_count;
     L.key_bits = 18;  // 6 bits per axis for 64 cells
 
-    launch_box(L, st);
+    // one launch up to the largest call (16 blocks of 4,096 agents), where the device has room
+    // for its cluster; else the general path
     uint32_t *skeys = nullptr, *perm = nullptr;
-    launch_sort(L, st, &skeys, &perm);
+    const bool one_launch = cluster_sort_shape(1, n, kNoallocMaxAgents, &L.cluster_blocks, &L.cluster_items);
+    if (one_launch) {
+        launch_cluster_sort(L, st, &skeys, &perm);
+    } else {
+        launch_box(L, st);
+        launch_sort(L, st, &skeys, &perm);
+    }
     float4 *pos_sorted = reinterpret_cast<float4 *>(scratch + kOffPos);
     GatherSet gs{};
     gs.src_f4[0] = L.pos;
@@ -186,9 +190,7 @@ extern "C" int tgpu_see_noalloc(const float *positions, unsigned n, const float 
     gs.nf4 = 1;
     launch_cell_table(L, skeys, 1, st, perm, &gs);  // and the positions into cell order
 
-    // the test model's see pass (agent_see alone): accumulators into the acc array
-    const KernelDesc &k = model_test_basic()->kernels[0];
-    float4 *acc = reinterpret_cast<float4 *>(scratch + kOffAcc);
+    // the test model's see pass (agent_see alone), its sums in the caller's order
     SeeLaunch S{};
     S.specs = L.specs;
     S.box = L.box;
@@ -205,15 +207,14 @@ extern "C" int tgpu_see_noalloc(const float *positions, unsigned n, const float 
     S.stage_cap = 0;
     S.stage_cells = 0;
     S.union_factor = 1;
+    S.rows = 1;
+    S.lanes = seer_lanes(n, kNoallocMates, 3, false);
     S.pairs = reinterpret_cast<unsigned long long *>(scratch + kOffPairs);
     S.telemetry = nullptr;
-    for (int c = 0; c < 4; ++c) {
-        S.io.in_f4[c] = c == 0 ? pos_sorted : acc;
-        S.io.out_f4[c] = c == 0 ? pos_sorted : acc;
-    }
-    k.launch_see(S, 0, st);
-    noalloc_unpermute_kernel<<<(n + 255) / 256, 256, 0, st>>>(perm, acc, reinterpret_cast<float4 *>(out), n);
-    launch_cell_table(L, skeys, 0, st);
+    S.io.in_f4[0] = pos_sorted;
+    S.io.out_f4[2] = reinterpret_cast<float4 *>(out);
+    S.io.in_u32[0] = perm;
+    launch_see_out(S, st);
     // launch errors first (only this call's: nothing was pending at entry), then the
     // errors of the work itself
     e = cudaGetLastError();
@@ -223,6 +224,7 @@ extern "C" int tgpu_see_noalloc(const float *positions, unsigned n, const float 
         snprintf(msg, sizeof(msg), "tgpu_see_noalloc: %s", cudaGetErrorString(e));
         return noalloc_fail(TGPU_ERR_CUDA, msg);
     }
+    if (one_launch) return TGPU_OK;  // (its sort waits for nothing that could run out)
     uint32_t err = 0;
     e = cudaMemcpy(&err, scratch + kOffErr, sizeof(err), cudaMemcpyDeviceToHost);
     if (e == cudaSuccess && err) {

@@ -111,6 +111,10 @@ uint32_t next_pow2(uint32_t v) {
 constexpr float kFill = 32.0f / 27.0f;
 constexpr uint32_t kFillAgents = 16384;
 
+// Largest segment that one launch sorts (a cluster of 8 blocks); larger ones take the
+// general path, which spreads them over more of the chip.
+constexpr uint32_t kClusterAgents = 16384;
+
 uint32_t log2u(uint32_t v) {
     uint32_t n = 0;
     while ((1u << n) < v) ++n;
@@ -246,33 +250,6 @@ int upload_contexts(TgpuBatch *b, int seg) {
     return TGPU_OK;
 }
 
-// Lanes per seer of a see pass over `seers` seers (row order).  With one lane per seer a
-// launch takes at least as long as one lane's walk, and needs enough seers to hide the
-// latency of its loads; below that the chip idles and several lanes share a seer's candidates
-// (see_group_kernel, which issues more instructions per candidate).  The longer a walk, the
-// more seers it takes: `mates` is the number of box-test passes a seer can expect from the
-// seen agents' mean density, and the size up to which 8 lanes win grows with about its cube
-// root.  Measured, us at 1 / 8 / 16 / 32 lanes, see pass (step where marked):
-//   SPH density, 512 mates:  2,048 seers 258 / 65 / 35 / 19, 20,480 433 / 129 / 98 / 84,
-//                            81,920 527 / 386 / 346 / 322, 262,144 1140 / 1162 / 1106 / 1062
-//   SPH force, list replay:  2,048 126 / 33 / 23 / 16, 20,480 147 / 57 / 56 / 67,
-//                            81,920 182 / 159 / 179 / 245, 131,072 233 / 264 / 298 / 400
-//   test model, 100 mates:   2,000 43 / 21 / 16 / 12, 12,000 53 / 24 / 26 / 33,
-//                            30,000 58 / 43 / 45 / 65, 50,000 62 / 63 / 71 / 102
-//   the same (step):  50 mates: 10,000 63 / 47 / 47 / 57, 40,000 72 / 70 / 83 / 117
-//                     25 mates: 5,000 53 / 43 / 43 / 48, 20,000 57 / 51 / 59 / 78, 40,000 61 / 65 / 81 / 116
-//                      4 mates: 10,000 49 / 45 / 49 / 59, 20,000 57 / 58 / 67 / 85
-//   two groups on a plane (step), 25 mates: 8,000 + 10,000 94 / 78 / 93 / 127, 16,000 each
-//                     97 / 92 / 122 / 179, 20,000 + 30,000 99 / 115 / 158 / 248
-uint32_t seer_lanes(uint64_t seers, double mates, int dims, bool replay) {
-    const double most = 9000.0 * pow(std::max(mates, 1.0), 0.37) * (dims < 3 ? 0.6 : 1.0);
-    if ((double)seers > most) return 1u;
-    if ((double)seers > most / 4.0) return 8u;
-    // a dense walk keeps 32 lanes busy row by row; a list of the same seer is shorter
-    if (mates >= 200.0 && !replay) return 32u;
-    return (double)seers > most / 16.0 ? 16u : 32u;
-}
-
 // The box-test passes an agent can expect among the agents of group `seen` if they were
 // spread evenly over their pushed extent (or fixed box).
 double expected_mates(const TgpuBatch *b, int seen, const float *radii) {
@@ -306,11 +283,38 @@ void set_lanes(TgpuBatch *b) {
     }
 }
 
+}  // namespace
+
+// Lanes per seer of a see pass over `seers` seers (row order).  With one lane per seer a
+// launch takes at least as long as one lane's walk, and needs enough seers to hide the
+// latency of its loads; below that the chip idles and several lanes share a seer's candidates
+// (see_group_kernel, which issues more instructions per candidate).  The longer a walk, the
+// more seers it takes: `mates` is the number of box-test passes a seer can expect from the
+// seen agents' mean density, and the size up to which 8 lanes win grows with about its cube
+// root.  Measured, us at 1 / 8 / 16 / 32 lanes, see pass (step where marked):
+//   SPH density, 512 mates:  2,048 seers 258 / 65 / 35 / 19, 20,480 433 / 129 / 98 / 84,
+//                            81,920 527 / 386 / 346 / 322, 262,144 1140 / 1162 / 1106 / 1062
+//   SPH force, list replay:  2,048 126 / 33 / 23 / 16, 20,480 147 / 57 / 56 / 67,
+//                            81,920 182 / 159 / 179 / 245, 131,072 233 / 264 / 298 / 400
+//   test model, 100 mates:   2,000 43 / 21 / 16 / 12, 12,000 53 / 24 / 26 / 33,
+//                            30,000 58 / 43 / 45 / 65, 50,000 62 / 63 / 71 / 102
+//   the same (step):  50 mates: 10,000 63 / 47 / 47 / 57, 40,000 72 / 70 / 83 / 117
+//                     25 mates: 5,000 53 / 43 / 43 / 48, 20,000 57 / 51 / 59 / 78, 40,000 61 / 65 / 81 / 116
+//                      4 mates: 10,000 49 / 45 / 49 / 59, 20,000 57 / 58 / 67 / 85
+//   two groups on a plane (step), 25 mates: 8,000 + 10,000 94 / 78 / 93 / 127, 16,000 each
+//                     97 / 92 / 122 / 179, 20,000 + 30,000 99 / 115 / 158 / 248
+uint32_t tgpu::seer_lanes(uint64_t seers, double mates, int dims, bool replay) {
+    const double most = 9000.0 * pow(std::max(mates, 1.0), 0.37) * (dims < 3 ? 0.6 : 1.0);
+    if ((double)seers > most) return 1u;
+    if ((double)seers > most / 4.0) return 8u;
+    // a dense walk keeps 32 lanes busy row by row; a list of the same seer is shorter
+    if (mates >= 200.0 && !replay) return 32u;
+    return (double)seers > most / 16.0 ? 16u : 32u;
+}
+
 // Per-segment grid bounds from the pushed agents: each axis gets a power-of-two cell
 // budget with 10% headroom over the pushed extent (bounded to 1024, the 10-bit Morton
 // limit); the dense table gets at most shared_megabytes of uint2 entries.
-}  // namespace
-
 int tgpu::prepare_specs(TgpuBatch *b) {
     if (!b->specs_dirty) return TGPU_OK;
     b->specs_dirty = false;
@@ -441,6 +445,7 @@ SortLaunch tgpu::sort_launch(TgpuBatch *b) {
     L.tiles = b->tiles;
     L.key_bits = b->key_bits;
     L.cluster_blocks = b->cluster_blocks;
+    L.cluster_items = b->cluster_items;
     return L;
 }
 
@@ -973,7 +978,7 @@ int alloc_batch(TgpuBatch *b) {
     b->ctx_stride = (std::max(m->see_ctx_bytes, m->act_ctx_bytes) + 15u) & ~15u;
     uint32_t largest = 0;
     for (const auto &sp : b->specs) largest = std::max(largest, sp.count);
-    b->cluster_blocks = cluster_sort_blocks((uint32_t)b->nseg, largest);
+    cluster_sort_shape((uint32_t)b->nseg, largest, kClusterAgents, &b->cluster_blocks, &b->cluster_items);
     return TGPU_OK;
 }
 

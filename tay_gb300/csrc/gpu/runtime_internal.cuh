@@ -68,7 +68,7 @@ struct TgpuBatch {
     std::vector<uint32_t> cta_begin;           // first CTA of each segment, + total
     std::vector<TgpuStatePass> state_passes;   // tgpu_state_create: the state's pass list
     uint32_t tiles = 0, ctas = 0, key_bits = 0;
-    uint32_t cluster_blocks = 0;  // SortLaunch::cluster_blocks
+    uint32_t cluster_blocks = 0, cluster_items = 0;  // SortLaunch::cluster_blocks, cluster_items
     bool specs_dirty = true;
     float fill = 0.0f;  // SegmentSpec::fill of every segment
 
@@ -128,6 +128,7 @@ namespace tgpu {
 
 // Runtime functions the adjoint module reuses.
 int prepare_specs(TgpuBatch *b);
+uint32_t seer_lanes(uint64_t seers, double mates, int dims, bool replay);
 void enqueue_step(TgpuBatch *b, const StepEvents *E = nullptr, bool write_through = false);
 // The batch's pair list on a see launch of run r, when r records or replays one.
 void attach_pair_list(const TgpuBatch *b, const KernelRun &r, SeeLaunch &S);

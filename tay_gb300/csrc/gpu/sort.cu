@@ -876,57 +876,62 @@ Scratch scratch_of(const SortLaunch &L) {
 
 namespace {
 
-// Agents a block of the cluster sort takes at most, and the largest segment it sorts: the
-// general path spreads larger ones over more of the chip.
-constexpr uint32_t kClusterChunk = 2048;
-constexpr uint32_t kClusterSegment = 16384;
-
-// The cluster sort of `items` agents a thread, launched (or, with `ask`, asked whether the
-// device can run its clusters).
+// The cluster sort, kItems agents a thread: its launch, or its attributes alone (`launch`
+// false).
 template <int kItems>
-cudaError_t cluster_sort(const SortLaunch &L, uint32_t blocks, cudaStream_t st, int *ask) {
+cudaError_t cluster_sort(const SortLaunch &L, bool launch, cudaStream_t st, int *clusters) {
+    auto *kernel = cluster_sort_kernel<kItems>;
     cudaLaunchAttribute attr;
     attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.x = blocks;
+    attr.val.clusterDim.x = L.cluster_blocks;
     attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
     cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(L.segments * blocks);
+    cfg.gridDim = dim3(L.segments * L.cluster_blocks);
     cfg.blockDim = dim3(kClusterThreads);
     cfg.dynamicSmemBytes = sizeof(ClusterSmem<kItems>);
     cfg.stream = st;
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
-    if (ask) {
-        cudaError_t e = cudaFuncSetAttribute(cluster_sort_kernel<kItems>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)sizeof(ClusterSmem<kItems>));
-        if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(ask, cluster_sort_kernel<kItems>, &cfg);
+    if (!launch) {
+        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(ClusterSmem<kItems>));
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+        if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(clusters, kernel, &cfg);
         return e;
     }
     uint32_t chunk_bits = 0;
     while ((1u << chunk_bits) < kItems * (uint32_t)kClusterThreads) ++chunk_bits;
-    return cudaLaunchKernelEx(&cfg, cluster_sort_kernel<kItems>, L.specs, L.pos, L.pos_max, L.box, L.grids, L.keys[1],
-                              L.vals[1], blocks, L.key_bits, (uint32_t)sort_digit_bits(L.key_bits), chunk_bits);
+    return cudaLaunchKernelEx(&cfg, kernel, L.specs, L.pos, L.pos_max, L.box, L.grids, L.keys[1], L.vals[1],
+                              L.cluster_blocks, L.key_bits, (uint32_t)sort_digit_bits(L.key_bits), chunk_bits);
+}
+cudaError_t cluster_sort(const SortLaunch &L, bool launch, cudaStream_t st, int *clusters) {
+    return L.cluster_items <= 2 ? cluster_sort<2>(L, launch, st, clusters) : cluster_sort<4>(L, launch, st, clusters);
 }
 
 }  // namespace
 
-uint32_t cluster_sort_blocks(uint32_t segments, uint32_t largest) {
-    if (!segments || largest > kClusterSegment) return 0u;
-    uint32_t blocks = 1;
-    while (blocks * kClusterChunk < largest) blocks *= 2;
-    if (segments * blocks > kClusterBlocks) return 0u;
+bool cluster_sort_shape(uint32_t segments, uint32_t largest, uint32_t most_agents, uint32_t *blocks, uint32_t *items) {
+    *blocks = 0;
+    *items = 0;
+    if (!segments || largest > most_agents) return false;
+    // 2 agents a thread up to 8 blocks (2,048 agents each), then 4
     SortLaunch L{};
     L.segments = segments;
+    L.cluster_items = largest <= 8u * 2u * kClusterThreads ? 2u : 4u;
+    L.cluster_blocks = 1;
+    while (L.cluster_blocks * L.cluster_items * kClusterThreads < largest) L.cluster_blocks *= 2;
+    if (L.cluster_blocks > kClusterMost || segments * L.cluster_blocks > kClusterWave) return false;
     int clusters = 0;
-    if (cluster_sort<kClusterChunk / kClusterThreads>(L, blocks, nullptr, &clusters) != cudaSuccess || clusters < 1) {
+    if (cluster_sort(L, false, nullptr, &clusters) != cudaSuccess || clusters < 1) {
         cudaGetLastError();
-        return 0u;
+        return false;
     }
-    return blocks;
+    *blocks = L.cluster_blocks;
+    *items = L.cluster_items;
+    return true;
 }
 
 void launch_cluster_sort(const SortLaunch &L, cudaStream_t st, uint32_t **sorted_keys, uint32_t **perm) {
-    cluster_sort<kClusterChunk / kClusterThreads>(L, L.cluster_blocks, st, nullptr);
+    cluster_sort(L, true, st, nullptr);
     *sorted_keys = L.keys[1];
     *perm = L.vals[1];
 }

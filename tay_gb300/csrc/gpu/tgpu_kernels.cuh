@@ -23,6 +23,7 @@ struct SortLaunch {
     uint32_t tiles;
     uint32_t key_bits;
     uint32_t cluster_blocks;   // blocks per segment of the one-launch sort (0: the general path)
+    uint32_t cluster_items;    // agents per thread of it: 2 or 4
 };
 
 struct GatherSet {
@@ -136,11 +137,12 @@ constexpr size_t sort_scratch_bytes(uint32_t segments, uint32_t tiles) {
 // Resets an extent accumulator (the pack kernel reduces the pushed positions into it).
 void reset_extent(BoxAcc *out, cudaStream_t st);
 void launch_sort(const SortLaunch &L, cudaStream_t st, uint32_t **sorted_keys, uint32_t **perm);
-// Boxes, grids, keys and sort of small segments in one launch (cluster_sort_kernel).
-// Blocks per segment it takes for `segments` segments of at most `largest` agents, 0 where the
-// general path (launch_box, launch_sort) does: larger segments, or more than one wave of them.
-constexpr uint32_t kClusterBlocks = 152;
-uint32_t cluster_sort_blocks(uint32_t segments, uint32_t largest);
+// Boxes, grids, keys and sort of small segments in one launch (cluster_sort_kernel), in place
+// of launch_box and launch_sort.  cluster_sort_shape: whether it takes `segments` segments of
+// at most `largest` agents (not more than most_agents, nor more blocks than one wave), and
+// with how many blocks per segment and agents per thread; also prepares its launch.
+constexpr uint32_t kClusterWave = 152;
+bool cluster_sort_shape(uint32_t segments, uint32_t largest, uint32_t most_agents, uint32_t *blocks, uint32_t *items);
 void launch_cluster_sort(const SortLaunch &L, cudaStream_t st, uint32_t **sorted_keys, uint32_t **perm);
 // Writes (write_runs = 1) or clears (0) the cell table of the sorted keys.  With `set`, the
 // same launch reorders its streams into cell order: dst[i] = src[perm[i]] for every agent.
