@@ -58,15 +58,13 @@ struct __align__(16) Term {
 
 template <class Acc>
 TGPU_D bool term_fn(const float4 &a, const float4 &b, const Acc &acc, uint32_t j, const Ctx &c, Term &t) {
-    const float dx = b.x - a.x, dy = b.y - a.y, dz = b.z - a.z;
-    float d2 = __fmul_rn(dx, dx);
-    d2 = __fadd_rn(d2, __fmul_rn(dy, dy));
-    d2 = __fadd_rn(d2, __fmul_rn(dz, dz));
+    const float3 d = see_detail::seen_minus_seer(a, b);
+    const float d2 = see_detail::length2(d);
     if (!(d2 < c.r2 && d2 > 0.0f)) return false;
     const float4 bv = acc.f4(1, j);
-    t.dx = dx;
-    t.dy = dy;
-    t.dz = dz;
+    t.dx = d.x;
+    t.dy = d.y;
+    t.dz = d.z;
     t.vx = bv.x;
     t.vy = bv.y;
     t.vz = bv.z;
@@ -94,25 +92,23 @@ TGPU_D void fold_fn(Seer &s, const Term &t) {
 // same order; through the term's registers the 1M-boid step measured 549 us instead of 534).
 template <class Acc>
 TGPU_D void see_fn(Seer &s, const float4 &a, const float4 &b, const Acc &acc, uint32_t j, const Ctx &c) {
-    const float dx = b.x - a.x, dy = b.y - a.y, dz = b.z - a.z;
-    float d2 = __fmul_rn(dx, dx);
-    d2 = __fadd_rn(d2, __fmul_rn(dy, dy));
-    d2 = __fadd_rn(d2, __fmul_rn(dz, dz));
+    const float3 d = see_detail::seen_minus_seer(a, b);
+    const float d2 = see_detail::length2(d);
     if (d2 < c.r2 && d2 > 0.0f) {
         const float4 bv = acc.f4(1, j);
         s.count += 1;
-        s.cx += dx;
-        s.cy += dy;
-        s.cz += dz;
+        s.cx += d.x;
+        s.cy += d.y;
+        s.cz += d.z;
         s.ax += bv.x;
         s.ay += bv.y;
         s.az += bv.z;
         if (d2 < c.sep_r2) {
             const float inv = __frcp_rn(d2);
             s.sep_count += 1;
-            s.sx -= __fmul_rn(dx, inv);
-            s.sy -= __fmul_rn(dy, inv);
-            s.sz -= __fmul_rn(dz, inv);
+            s.sx -= __fmul_rn(d.x, inv);
+            s.sy -= __fmul_rn(d.y, inv);
+            s.sz -= __fmul_rn(d.z, inv);
         }
     }
 }
@@ -120,10 +116,8 @@ TGPU_D void see_fn(Seer &s, const float4 &a, const float4 &b, const Acc &acc, ui
 // The pairs see_fn acts on: 0 < d2 < r2, d2 rounded exactly as see_fn rounds it (the walk
 // enters the see body only for these).
 TGPU_D bool keep_fn(const float4 &a, const float4 &b, const Ctx &c) {
-    const float dx = b.x - a.x, dy = b.y - a.y, dz = b.z - a.z;
-    float d2 = __fmul_rn(dx, dx);
-    d2 = __fadd_rn(d2, __fmul_rn(dy, dy));
-    d2 = __fadd_rn(d2, __fmul_rn(dz, dz));
+    const float3 d = see_detail::seen_minus_seer(a, b);
+    const float d2 = see_detail::length2(d);
     return d2 < c.r2 && d2 > 0.0f;
 }
 

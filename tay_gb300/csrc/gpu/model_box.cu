@@ -52,7 +52,8 @@ struct See {
     template <class Acc>
     TGPU_D static bool term(const Seer &, const float4 &a, const float4 &b, const Acc &, uint32_t, const SeeCtx &,
                             Term &t) {
-        t = {b.x - a.x, b.y - a.y, b.z - a.z};
+        const float3 d = see_detail::seen_minus_seer(a, b);
+        t = {d.x, d.y, d.z};
         return true;
     }
     TGPU_D static void fold(Seer &s, const Term &t, const SeeCtx &) { fold_fn(s, t); }

@@ -45,11 +45,13 @@ TGPU_D void fold_fn(Seer &s, const Term &t) {
 struct See {
     using Term = test_basic::Term;
     static constexpr bool kCheapTerm = true;
+    static constexpr int kLaneUnroll = 4;  // (100,000 agents: see pass 60 us at 2, 43 at 4, 46 at 8)
     static constexpr bool kSeenMinusSeer = true;  // d = b - a
     template <class Acc>
     TGPU_D static bool term(const Seer &, const float4 &a, const float4 &b, const Acc &, uint32_t, const SeeCtx &,
                             Term &t) {
-        t = {b.x - a.x, b.y - a.y, b.z - a.z};
+        const float3 d = see_detail::seen_minus_seer(a, b);
+        t = {d.x, d.y, d.z};
         return true;
     }
     TGPU_D static void fold(Seer &s, const Term &t, const SeeCtx &) { fold_fn(s, t); }

@@ -220,6 +220,31 @@ struct SeenMinusSeerOf<P, decltype((void)P::kSeenMinusSeer)> {
     static constexpr bool value = P::kSeenMinusSeer;
 };
 
+// Whether P's terms cost next to nothing and read nothing but the position (P::kCheapTerm):
+// they are computed where a candidate is tested.  Others are computed for the candidates that
+// passed, gathered until they fill the lanes.
+template <class P, class = void>
+struct CheapOf {
+    static constexpr bool value = false;
+};
+template <class P>
+struct CheapOf<P, decltype((void)P::kCheapTerm)> {
+    static constexpr bool value = P::kCheapTerm;
+};
+
+// seen - seer, x and y in one packed subtraction (each half rounded as the scalar one; the
+// seer's negated pair stays in registers).
+TGPU_D float3 seen_minus_seer(const float4 &a, const float4 &b) {
+    const float2 xy = __fadd2_rn(make_float2(b.x, b.y), make_float2(-a.x, -a.y));
+    return make_float3(xy.x, xy.y, b.z - a.z);
+}
+
+// The square of a difference's length, each product and sum rounded separately.
+TGPU_D float length2(const float3 &d) {
+    const float2 m = __fmul2_rn(make_float2(d.x, d.y), make_float2(d.x, d.y));
+    return __fadd_rn(__fadd_rn(m.x, m.y), __fmul_rn(d.z, d.z));
+}
+
 // A kept candidate into the recorder's list (the gated walk counts box-test passes itself).
 TGPU_D void record_kept(ListRec &r, uint32_t j) {
     if (r.n < r.cap) reinterpret_cast<uint32_t *>(r.idx)[((size_t)(r.n >> 2) * r.stride + r.seer) * 4u + (r.n & 3u)] = j;
@@ -236,13 +261,24 @@ TGPU_D void lane_one(typename P::Seer &s, const float4 &sp, const float4 &b, con
         // the reference's test on d = seer - seen, computed in the direction the model's keep
         // and see use (|seen - seer| is the same float), so the compiler shares it
         bool hit;
-        if constexpr (SeenMinusSeerOf<P>::value)
-            hit = !(fabsf(b.x - sp.x) > r4.x) && !(fabsf(b.y - sp.y) > r4.y) && !(fabsf(b.z - sp.z) > r4.z);
-        else
+        if constexpr (SeenMinusSeerOf<P>::value) {
+            const float3 d = seen_minus_seer(sp, b);
+            hit = !(fabsf(d.x) > r4.x) && !(fabsf(d.y) > r4.y) && !(fabsf(d.z) > r4.z);
+        } else {
             hit = !(fabsf(sp.x - b.x) > r4.x) && !(fabsf(sp.y - b.y) > r4.y) && !(fabsf(sp.z - b.z) > r4.z);
+        }
         pairs += hit ? 1u : 0u;
         if (hit && (SelfSafeOf<P>::value || j != self) && P::keep(sp, b, sctx)) {
             if constexpr (kRec) record_kept(*rec, j);
+            P::see(s, sp, b, acc, j, sctx);
+        }
+    } else if constexpr (SeenMinusSeerOf<P>::value && CheapOf<P>::value && !kRec) {
+        // a body of a few additions on the same difference: no branch
+        const float3 d = seen_minus_seer(sp, b);
+        const bool hit = (int)!(fabsf(d.x) > r4.x) & (int)!(fabsf(d.y) > r4.y) & (int)!(fabsf(d.z) > r4.z) &
+                         (int)(j != self);
+        if (hit) {
+            ++pairs;
             P::see(s, sp, b, acc, j, sctx);
         }
     } else {
@@ -993,18 +1029,6 @@ struct TermsOf<P, std::void_t<typename P::Term>> {
     static constexpr bool value = true;
 };
 
-// Whether P's terms cost next to nothing and read nothing but the position (P::kCheapTerm):
-// they are computed where a candidate is tested.  Others are computed for the candidates that
-// passed, gathered until they fill the lanes.
-template <class P, class = void>
-struct CheapOf {
-    static constexpr bool value = false;
-};
-template <class P>
-struct CheapOf<P, decltype((void)P::kCheapTerm)> {
-    static constexpr bool value = P::kCheapTerm;
-};
-
 // Slots of a seer's queue: two chunks add at most 2 G to what the last ones left.
 constexpr int group_slots(int g) { return g > 8 ? 4 * g : 32; }
 
@@ -1049,10 +1073,9 @@ TGPU_D void eval_terms(typename P::Seer &s, const float4 &sp, bool take, uint32_
 // The box test without branches, on the difference the pass's own functions compute.
 template <class P>
 TGPU_D bool box_hit_flat(const float4 &a, const float4 &b, const float4 &r) {
-    constexpr bool kSeenFirst = SeenMinusSeerOf<P>::value;
-    const float dx = kSeenFirst ? b.x - a.x : a.x - b.x, dy = kSeenFirst ? b.y - a.y : a.y - b.y,
-                dz = kSeenFirst ? b.z - a.z : a.z - b.z;
-    return (int)!(fabsf(dx) > r.x) & (int)!(fabsf(dy) > r.y) & (int)!(fabsf(dz) > r.z);
+    const float3 d = SeenMinusSeerOf<P>::value ? seen_minus_seer(a, b)
+                                               : make_float3(a.x - b.x, a.y - b.y, a.z - b.z);
+    return (int)!(fabsf(d.x) > r.x) & (int)!(fabsf(d.y) > r.y) & (int)!(fabsf(d.z) > r.z);
 }
 
 }  // namespace see_detail
