@@ -36,6 +36,8 @@ struct KernelDesc {
                                        // passes of one group accumulate); 0: starts from zero
     int pair_list;                     // 1: can record a pair list for the next see pass (P::keep);
                                        // 2: can replay the previous pass's list (P::replay_ok)
+    int packs;                         // pair_list 1: the pass also writes, per agent, the 32 bytes the
+                                       // replaying pass reads of a neighbour (io slot nf4; P::kPack there)
 };
 
 // A supported pass sequence: the func names in registration order, and the kernels

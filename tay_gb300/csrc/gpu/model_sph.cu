@@ -26,7 +26,9 @@
 namespace tgpu {
 namespace sph {
 
-enum { POS = 0, VEL = 1, RP = 2, ACC = 3 };
+// PACK: what the force pass reads of a neighbour, 32 bytes {x, y, z, P / rho^2, v.xyz, rho},
+// written by a density pass that records its pairs (null when it does not).
+enum { POS = 0, VEL = 1, RP = 2, ACC = 3, PACK = 4 };
 enum { ID = 0 };
 
 struct Ctx {
@@ -120,10 +122,16 @@ struct Density {
         Term t;
         if (term(s, a, b, acc, j, c, t)) fold(s, t, c);
     }
-    TGPU_D static void finish(Seer &s, const float4 &, const PassIO &io, uint32_t i, const Ctx &c, const Ctx &) {
+    TGPU_D static void finish(Seer &s, const float4 &a, const PassIO &io, uint32_t i, const Ctx &c, const Ctx &) {
         const float P = kPressure ? pressure(s.rho, c) : 0.0f;
         // A = P / rho^2, the pressure term every pair of the force pass needs
-        io.out_f4[RP][i] = make_float4(s.rho, P, P / (s.rho * s.rho), 0.0f);
+        const float A = P / (s.rho * s.rho);
+        io.out_f4[RP][i] = make_float4(s.rho, P, A, 0.0f);
+        if (kPressure && io.out_f4[PACK]) {
+            const float4 v = io.in_f4[VEL][i];
+            io.out_f4[PACK][2 * (size_t)i] = make_float4(a.x, a.y, a.z, A);
+            io.out_f4[PACK][2 * (size_t)i + 1] = make_float4(v.x, v.y, v.z, s.rho);
+        }
     }
 };
 
@@ -146,6 +154,9 @@ struct Force {
     // every pair this see function acts on (r2 < support2, r2 > 0) when the support is not
     // wider here; for the other candidates the see function does nothing
     static constexpr int kPairList = 2;
+    // A replayed neighbour is one 32-byte load.  Reading position, velocity and {rho, P, A} as
+    // three streams kept L1 busy with three scattered 16-byte accesses a pair.
+    static constexpr int kPack = PACK;
     TGPU_D static bool replay_ok(const Ctx &mine, const Ctx &rec) { return mine.support2 <= rec.support2; }
     // when it walks: the see body runs only for 0 < r2 < support2
     static constexpr bool kKeepGate = true;
@@ -171,8 +182,18 @@ struct Force {
         const float dx = a.x - b.x, dy = a.y - b.y, dz = a.z - b.z;
         const float r2 = dist2(dx, dy, dz);
         if (!(r2 < c.support2 && r2 > 0.0f)) return false;
-        const float4 bv = acc.f4(1, j);
-        const float4 brp = acc.f4(2, j);
+        float4 bv;
+        float brho, bA;
+        if constexpr (std::is_same_v<Acc, see_detail::PackedSeen>) {
+            bv = acc.hi;
+            brho = acc.hi.w;
+            bA = acc.lo.w;
+        } else {
+            const float4 brp = acc.f4(2, j);
+            bv = acc.f4(1, j);
+            brho = brp.x;
+            bA = brp.z;
+        }
         // 1/r from one correctly rounded reciprocal square root, r = r2 * (1/r), dw / r
         // as a product, and the viscosity term's two divisions as one
         const float inv_r = __frsqrt_rn(r2);
@@ -183,10 +204,10 @@ struct Force {
         const float vr = __fmaf_rn(vz, dz, __fmaf_rn(vy, dy, vx * dx));
         float visc = 0.0f;
         if (vr < 0.0f) {
-            const float rho_bar = 0.5f * (s.rho + brp.x);
+            const float rho_bar = 0.5f * (s.rho + brho);
             visc = -(c.alpha * c.c0 * (c.h * vr)) / ((r2 + c.eta2) * rho_bar);
         }
-        t.coef = -c.m * ((s.A + brp.z) + visc) * (dw * inv_r);
+        t.coef = -c.m * ((s.A + bA) + visc) * (dw * inv_r);
         t.dx = dx;
         t.dy = dy;
         t.dz = dz;
@@ -259,7 +280,7 @@ const KernelDesc kKernels[] = {
     {"sph_density", nullptr, bit(RP), 0, bit(POS), 1, launch_see_t<Density<false>>, nullptr,
      prepare_see_t<Density<false>>, 0, 0},
     {"sph_density", "sph_pressure", bit(RP), 0, bit(POS), 1, launch_see_t<Density<true>>, nullptr,
-     prepare_see_t<Density<true>>, 0, 1},
+     prepare_see_t<Density<true>>, 0, 1, 1},
     {"sph_force", nullptr, bit(ACC), 0, bit(POS) | bit(VEL) | bit(RP), 3, launch_see_t<Force<false>>, nullptr,
      prepare_see_t<Force<false>>, 0, 2},
     {"sph_force", "sph_integrate", bit(POS) | bit(VEL), 0, bit(POS) | bit(VEL) | bit(RP), 3,

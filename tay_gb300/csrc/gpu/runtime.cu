@@ -150,6 +150,7 @@ void free_batch(TgpuBatch *b) {
     cudaFree(b->d_aos);
     cudaFree(b->plist_idx);
     cudaFree(b->plist_count);
+    cudaFree(b->pack);
     for (auto &r : b->runs) {
         cudaFree(r.d_radii);
         cudaFree(r.d_see_ctx);
@@ -495,6 +496,10 @@ void tgpu::attach_pair_list(const TgpuBatch *b, const KernelRun &r, SeeLaunch &S
         S.plist.rec_ctx = b->runs[r.list_src].d_see_ctx;
         S.lanes = r.replay_lanes;
     }
+    if (b->pack) {
+        S.io.out_f4[b->m->nf4] = b->pack;
+        S.io.in_f4[b->m->nf4] = b->pack;
+    }
 }
 
 void tgpu::enqueue_step(TgpuBatch *b, const StepEvents *E, bool write_through) {
@@ -666,6 +671,7 @@ unsigned long long tgpu_batch_device_bytes(const TgpuBatch *b) {
     bytes += b->table_entries * sizeof(uint2);
     bytes += n * b->m->agent_bytes;
     if (b->plist_idx) bytes += n * (4ull * b->plist_cap + sizeof(uint2));
+    if (b->pack) bytes += n * 2ull * sizeof(float4);
     return bytes;
 }
 
@@ -796,7 +802,8 @@ int tgpu_register_model(const void *desc, unsigned abi) {
         const KernelDesc &d = m->kernels[k];
         const bool ok = d.see ? (d.launch_see && d.prepare) : (d.act && d.launch_act);
         if (!ok || (d.writes_f4 & ~all_f4) || (d.seen_f4 & ~all_f4) || (d.writes_u32 & ~all_u32) ||
-            d.staged_f4 < 0 || d.staged_f4 > kMaxF4 || d.pair_list < 0 || d.pair_list > 2)
+            d.staged_f4 < 0 || d.staged_f4 > kMaxF4 || d.pair_list < 0 || d.pair_list > 2 ||
+            (d.packs && (d.pair_list != 1 || m->nf4 >= kMaxF4)))
             return fail(TGPU_ERR_ARG, "model '%s': kernel %d is incomplete or names streams it does not have", m->name, k);
     }
     for (int p = 0; p < m->nprograms; ++p) {
@@ -1039,6 +1046,9 @@ int setup_pair_lists(TgpuBatch *b) {
     b->plist_cap = cap;
     CKR(cudaMalloc(&b->plist_idx, (size_t)(cap / 4u) * b->total * sizeof(uint4)));
     CKR(cudaMalloc(&b->plist_count, (size_t)b->total * sizeof(uint2)));
+    bool packs = false;
+    for (const auto &r : b->runs) packs = packs || (r.list_mode == 1u && r.k->packs);
+    if (packs) CKR(cudaMalloc(&b->pack, 2 * (size_t)b->total * sizeof(float4)));
     return TGPU_OK;
 }
 

@@ -103,6 +103,7 @@ struct TgpuBatch {
     uint4 *plist_idx = nullptr;
     uint2 *plist_count = nullptr;
     uint32_t plist_cap = 0;
+    float4 *pack = nullptr;  // [2 * total] the neighbour data a recording pass packs (KernelDesc::packs)
 
     cudaStream_t st = nullptr;
     cudaEvent_t e0 = nullptr, e1 = nullptr;

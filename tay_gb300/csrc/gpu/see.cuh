@@ -120,6 +120,26 @@ struct ListOf<P, decltype((void)P::kPairList)> {
     static constexpr int value = P::kPairList;
 };
 
+// What a replaying pass reads of a neighbour, packed into 32 consecutive bytes by the pass
+// that recorded the list (P::kPack: the io slot of both, two float4 per agent); absent: -1.
+template <class P, class = void>
+struct PackOf {
+    static constexpr int value = -1;
+};
+template <class P>
+struct PackOf<P, decltype((void)P::kPack)> {
+    static constexpr int value = P::kPack;
+};
+// One neighbour's packed 32 bytes, in one load; lo's x, y, z are its position.
+struct PackedSeen {
+    float4 lo, hi;
+    TGPU_D PackedSeen(const float4 *pack, uint32_t j) {
+        asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+            : "=f"(lo.x), "=f"(lo.y), "=f"(lo.z), "=f"(lo.w), "=f"(hi.x), "=f"(hi.y), "=f"(hi.z), "=f"(hi.w)
+            : "l"(pack + 2 * (size_t)j));
+    }
+};
+
 // The walk of a pass that records no pair list.
 struct NoRec {};
 
@@ -325,28 +345,32 @@ TGPU_D void lane_run(typename P::Seer &s, const float4 &sp, const float4 &r4, ui
 }
 
 // Replay of a recorded pair list: the see function over the seer's n entries in their
-// recorded order, one group of four per load, two positions loaded ahead; words past the
-// n-th are never used; the seer itself is skipped when the pass skips self.
+// recorded order, one group of four per load, two neighbours loaded ahead; words past the
+// n-th are never used; the seer itself is skipped when the pass skips self.  `pack`: the
+// neighbours' packed data of a pass with P::kPack.
 template <class P, class Acc>
 TGPU_D void list_run(typename P::Seer &s, const float4 &sp, const PairList &pl, uint32_t i, uint32_t n, uint32_t self,
-                     const float4 *pos, const Acc &acc, const typename P::SeeCtx &sctx) {
+                     const float4 *pos, const Acc &acc, const float4 *pack, const typename P::SeeCtx &sctx) {
     const uint4 *e = pl.idx + i;
     const size_t stride = pl.stride;
+    // entries j0 and, with `two`, j1
+    auto pair = [&](uint32_t j0, uint32_t j1, bool two) {
+        if constexpr (PackOf<P>::value >= 0) {
+            const PackedSeen b0(pack, j0), b1(pack, two ? j1 : j0);
+            if (j0 != self) P::see(s, sp, b0.lo, b0, j0, sctx);
+            if (two && j1 != self) P::see(s, sp, b1.lo, b1, j1, sctx);
+        } else {
+            const float4 b0 = __ldg(pos + j0);
+            const float4 b1 = two ? __ldg(pos + j1) : b0;
+            if (j0 != self) P::see(s, sp, b0, acc, j0, sctx);
+            if (two && j1 != self) P::see(s, sp, b1, acc, j1, sctx);
+        }
+    };
     for (uint32_t t = 0; t < n; t += 4) {
         const uint4 g = __ldg(e + (size_t)(t >> 2) * stride);
         const uint32_t m = n - t;  // entries of this group: min(m, 4)
-        {
-            const float4 b0 = __ldg(pos + g.x);
-            const float4 b1 = m > 1u ? __ldg(pos + g.y) : b0;
-            if (g.x != self) P::see(s, sp, b0, acc, g.x, sctx);
-            if (m > 1u && g.y != self) P::see(s, sp, b1, acc, g.y, sctx);
-        }
-        if (m > 2u) {
-            const float4 b2 = __ldg(pos + g.z);
-            const float4 b3 = m > 3u ? __ldg(pos + g.w) : b2;
-            if (g.z != self) P::see(s, sp, b2, acc, g.z, sctx);
-            if (m > 3u && g.w != self) P::see(s, sp, b3, acc, g.w, sctx);
-        }
+        pair(g.x, g.y, m > 1u);
+        if (m > 2u) pair(g.z, g.w, m > 3u);
     }
 }
 
@@ -790,7 +814,8 @@ __global__ void __launch_bounds__(kSeeThreads, kStage ? 1 : 8) see_rows_kernel(S
             replayed = __all_sync(0xffffffffu, covers && c.x <= L.plist.cap);
             if (replayed && L.telemetry && lane == 0) atomicAdd(L.telemetry + 5, 1ull);
             if (replayed && active) {
-                list_run<P>(s, sp, L.plist, i, c.x, self, pos, acc, sctx);
+                const float4 *pack = PackOf<P>::value >= 0 ? L.io.in_f4[PackOf<P>::value < 0 ? 0 : PackOf<P>::value] : nullptr;
+                list_run<P>(s, sp, L.plist, i, c.x, self, pos, acc, pack, sctx);
                 // the walk's count: box-test passes with every other agent, and the seer
                 // itself unless the pass skips it
                 pairs += c.y + ((!L.skip_self && box_hit(sp, sp, r4)) ? 1u : 0u);
@@ -1059,12 +1084,19 @@ TGPU_D void fold_terms(typename P::Seer &s, const typename P::Term *q, uint32_t 
 }
 
 // The terms of up to G candidates of a seer, one a lane (those with `take`), folded in lane
-// order.
-template <class P, int G, class Acc>
+// order; kPacked: read from `pos` as packed neighbours.
+template <class P, int G, bool kPacked = false, class Acc>
 TGPU_D void eval_terms(typename P::Seer &s, const float4 &sp, bool take, uint32_t j, const float4 *pos,
                        const Acc &acc, typename P::Term *q, const Group<G> &gr, const typename P::SeeCtx &c) {
     typename P::Term t;
-    if (take) take = P::term(s, sp, __ldg(pos + j), acc, j, c, t);
+    if (take) {
+        if constexpr (kPacked) {
+            const PackedSeen b(pos, j);
+            take = P::term(s, sp, b.lo, b, j, c, t);
+        } else {
+            take = P::term(s, sp, __ldg(pos + j), acc, j, c, t);
+        }
+    }
     const uint32_t v = gr.votes(take);
     if (take) q[__popc(v & gr.below)] = t;
     fold_terms<P, G>(s, q, (uint32_t)__popc(v), c);
@@ -1179,7 +1211,11 @@ __global__ void __launch_bounds__(kSeeThreads, 8) see_group_kernel(SeeLaunch L) 
                 for (uint32_t t = sub; __any_sync(0xffffffffu, t - sub < c.x); t += G) {
                     const uint32_t f = t + G;
                     const uint32_t next = f < c.x ? __ldg(e + (size_t)(f >> 2) * stride + (f & 3u)) : self;
-                    eval_terms<P, G>(s, sp, t < c.x && j != self, j, pos, acc, terms, gr, sctx);
+                    if constexpr (PackOf<P>::value >= 0)
+                        eval_terms<P, G, true>(s, sp, t < c.x && j != self, j, L.io.in_f4[PackOf<P>::value], acc,
+                                               terms, gr, sctx);
+                    else
+                        eval_terms<P, G>(s, sp, t < c.x && j != self, j, pos, acc, terms, gr, sctx);
                     j = next;
                 }
                 if (sub == 0 && active) pairs += c.y + ((!L.skip_self && box_hit(sp, sp, r4)) ? 1u : 0u);
