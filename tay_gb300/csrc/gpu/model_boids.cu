@@ -121,17 +121,18 @@ TGPU_D bool keep_fn(const float4 &a, const float4 &b, const Ctx &c) {
     return d2 < c.r2 && d2 > 0.0f;
 }
 
+// Lengths in the act.  A sum of two products may be fused either way, and copies of the act in
+// different kernels did round differently, so the order is spelled out: x's product fused onto
+// y's, or, for a steering vector (steer), y's onto x's, as the walk with one lane per seer has
+// always rounded them.
 TGPU_D float len3(float x, float y, float z) {
-    float s = x * x;
-    s = s + y * y;
-    s = s + z * z;
-    return sqrtf(s);
+    return sqrtf(__fmaf_rn(z, z, __fmaf_rn(x, x, __fmul_rn(y, y))));
 }
 
 TGPU_D void steer(float vx, float vy, float vz, int n, float w, const float4 &v, const Ctx &c, float &ax, float &ay,
                   float &az) {
     if (n <= 0) return;
-    const float len = len3(vx, vy, vz);
+    const float len = sqrtf(__fmaf_rn(vz, vz, __fmaf_rn(vy, vy, __fmul_rn(vx, vx))));
     if (!(len > 0.0f)) return;
     const float k = c.max_speed / len;
     float sx = vx * k - v.x, sy = vy * k - v.y, sz = vz * k - v.z;

@@ -23,6 +23,9 @@ def _records(model, n):
     if model == "boids":  # 64 neighbours inside the box, both halves of the separation test
         ps = W.basic_points(n, seed=93, side=(125.0 * n) ** (1 / 3))
         return M.boids_setup(r=10.0, part=10.0), M.records(M.BOIDS_RECORD, ps.p, ps.v)
+    if model == "flock":  # scattered: a few neighbours, or none
+        ps = W.boids_points(n, seed=97)
+        return M.boids_setup(r=10.0, part=10.0), M.records(M.BOIDS_RECORD, ps.p, ps.v)
     if model == "heap":  # every particle inside every other's support: the pair lists overflow
         p = np.full((n, 4), 0.05, np.float32)
         p[:, :3] += np.random.default_rng(94).uniform(0, 0.01, (n, 3)).astype(np.float32)
@@ -52,7 +55,7 @@ def _run(setup, recs, steps, **tuning):
 @pytest.mark.parametrize("model,n", [
     ("test", 1), ("test", 2), ("test", 127), ("test", 129), ("test", 2500), ("test", 4097), ("test", 12289),
     ("test", 40000), ("test", 60001), ("box", 3), ("box", 3001), ("box", 12289), ("boids", 33), ("boids", 2049),
-    ("boids", 8193), ("boids", 30001), ("sph", 5), ("sph", 4097), ("sph", 20001), ("sph", 40001), ("sph", 130000),
+    ("boids", 8193), ("boids", 30001), ("flock", 600), ("flock", 5000), ("sph", 5), ("sph", 4097), ("sph", 20001), ("sph", 40001), ("sph", 130000),
     ("heap", 700)])
 def test_shared_lanes_equal_one_lane(gpu, model, n):
     setup, recs = _records(model, n)
