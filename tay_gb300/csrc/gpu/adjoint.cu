@@ -23,7 +23,7 @@
 namespace tgpu {
 namespace {
 
-enum { A_POS = 0, A_VEL = 1, A_RP = 2, A_ABAR = 3, A_XBAR = 4, A_VBAR = 5, A_RHOBAR = 6, A_THETA = 7 };
+enum { A_POS = 0, A_VEL = 1, A_RP = 2, A_ABAR = 3, A_XBAR = 4, A_VBAR = 5, A_RHOBAR = 6, A_THETA = 7, A_PACK = 6 };
 constexpr int SPH_POS = 0, SPH_VEL = 1, SPH_RP = 2, SPH_ACC = 3, SPH_ID = 0;
 
 struct Record {
@@ -56,17 +56,19 @@ __global__ void __launch_bounds__(kSortThreads) gid_kernel(const SegmentSpec *__
     for (uint32_t i = beg + threadIdx.x; i < end; i += kSortThreads) gid[i] = s.begin + id[i];
 }
 
-// Per-segment sum of the particles' parameter gradients, in a fixed order: one block per
-// segment, each thread a strided partial sum, then a shared-memory tree.
+// Per-segment sum of the particles' parameter gradients (each already summed over the
+// steps), in a fixed order: one block per segment, each thread a strided partial sum, then
+// a shared-memory tree.  Once per backward sweep: summed every step it took 11 us of double
+// additions on one SM per segment.
 __global__ void __launch_bounds__(256) theta_reduce_kernel(const SegmentSpec *__restrict__ specs,
-                                                           const float4 *__restrict__ theta, double *__restrict__ acc) {
+                                                           const double2 *__restrict__ theta, double *__restrict__ out) {
     __shared__ double sa[256], sc[256];
     const SegmentSpec s = specs[blockIdx.x];
     double a = 0.0, c = 0.0;
-    for (uint32_t i = s.begin + threadIdx.x; i < s.begin + s.count; i += 256) {
-        const float4 t = theta[i];
-        a += (double)t.x;
-        c += (double)t.y;
+    for (uint32_t i = threadIdx.x; i < s.count; i += 256) {
+        const double2 t = theta[s.begin + i];
+        a += t.x;
+        c += t.y;
     }
     sa[threadIdx.x] = a;
     sc[threadIdx.x] = c;
@@ -79,8 +81,8 @@ __global__ void __launch_bounds__(256) theta_reduce_kernel(const SegmentSpec *__
         __syncthreads();
     }
     if (threadIdx.x == 0) {
-        acc[2 * blockIdx.x] += sa[0];
-        acc[2 * blockIdx.x + 1] += sc[0];
+        out[2 * blockIdx.x] = sa[0];
+        out[2 * blockIdx.x + 1] = sc[0];
     }
 }
 
@@ -99,6 +101,7 @@ struct TgpuAdjoint {
     std::vector<tgpu::StepList> lists;
     float4 *xbar_id = nullptr, *vbar_id = nullptr, *xbar_s = nullptr, *vbar_s = nullptr;
     float4 *abar = nullptr, *rhobar = nullptr, *theta = nullptr;
+    double2 *theta_id = nullptr;  // per particle (id order): gradients summed over the steps
     double *d_theta = nullptr;
     std::vector<void *> allocs;
     size_t bytes = 0;
@@ -274,6 +277,7 @@ void backward_step(TgpuAdjoint *a, const Record &r, const StepList *pl = nullptr
     ia.out_f4[A_XBAR] = a->xbar_s;
     ia.in_f4[A_VBAR] = a->vbar_id;
     ia.out_f4[A_VBAR] = a->vbar_s;
+    if (pl) ia.out_f4[A_PACK] = b->pack;  // what the replaying force adjoint reads of a neighbour
     const KernelRun &rd = b->runs[0];
     const KernelRun &rf = b->runs[1];
     ActLaunch A{};
@@ -289,12 +293,15 @@ void backward_step(TgpuAdjoint *a, const Record &r, const StepList *pl = nullptr
     fa.in_f4[A_ABAR] = fa.out_f4[A_ABAR] = a->abar;
     fa.in_f4[A_XBAR] = fa.out_f4[A_XBAR] = a->xbar_s;
     fa.in_f4[A_VBAR] = fa.out_f4[A_VBAR] = a->vbar_s;
-    fa.in_f4[A_RHOBAR] = fa.out_f4[A_RHOBAR] = a->rhobar;
+    fa.out_f4[A_RHOBAR] = a->rhobar;
     fa.in_f4[A_THETA] = fa.out_f4[A_THETA] = a->theta;
     // the force adjoint records the step's pairs for the density adjoint when the batch
     // keeps pair lists for its forward passes (the same cell order and walk conditions)
     SeeLaunch F = see_launch(b, rf, fa);
-    SeeLaunch D = see_launch(b, rd, fa);
+    if (pl) F.io.in_f4[A_PACK] = b->pack;
+    PassIO da = fa;
+    da.in_f4[A_POS] = a->rhobar;
+    SeeLaunch D = see_launch(b, rd, da);
     D.skip_self = 1;  // the self pair contributes nothing to the density adjoint
     if (pl) {
         // the forward density pass's list: it holds every pair inside the support (and the
@@ -319,9 +326,10 @@ void backward_step(TgpuAdjoint *a, const Record &r, const StepList *pl = nullptr
     sa.out_f4[A_XBAR] = a->xbar_id;
     sa.in_f4[A_VBAR] = a->vbar_s;
     sa.out_f4[A_VBAR] = a->vbar_id;
+    sa.in_f4[A_THETA] = a->theta;
+    sa.out_f4[A_THETA] = reinterpret_cast<float4 *>(a->theta_id);
     A.io = sa;
     a->K->scatter_adj(A, st);
-    theta_reduce_kernel<<<b->nseg, 256, 0, st>>>(b->d_specs, a->theta, a->d_theta);
     launch_cell_table(L, r.keys, 0, st);
 }
 
@@ -376,6 +384,7 @@ int tgpu_adjoint_create(TgpuBatch *b, int steps, int checkpoint_every, int keep_
     if (!rc) rc = alloc(a, &a->abar, n);
     if (!rc) rc = alloc(a, &a->rhobar, n);
     if (!rc) rc = alloc(a, &a->theta, n);
+    if (!rc) rc = alloc(a, &a->theta_id, n);
     if (!rc) rc = alloc(a, &a->d_theta, 2 * (size_t)b->nseg);
     // per-step lists of one segment when the batch pairs its density and force passes
     // through a list (checkpoint mode only: a list per step of the whole rollout would not fit)
@@ -440,7 +449,7 @@ int tgpu_adjoint_backward(TgpuAdjoint *a, const float *dl_dpos, const float *dl_
     cudaMemsetAsync(a->vbar_id, 0, n * sizeof(float4), st);
     if (dl_dpos) cudaMemcpyAsync(a->xbar_id, dl_dpos, n * sizeof(float4), cudaMemcpyHostToDevice, st);
     if (dl_dvel) cudaMemcpyAsync(a->vbar_id, dl_dvel, n * sizeof(float4), cudaMemcpyHostToDevice, st);
-    cudaMemsetAsync(a->d_theta, 0, 2 * (size_t)b->nseg * sizeof(double), st);
+    cudaMemsetAsync(a->theta_id, 0, n * sizeof(double2), st);
     cudaEventRecord(a->e0, st);
     if (a->every == 0) {
         for (int s = a->steps - 1; s >= 0; --s) backward_step(a, a->rec[s]);
@@ -467,6 +476,7 @@ int tgpu_adjoint_backward(TgpuAdjoint *a, const float *dl_dpos, const float *dl_
         // lists over the last segment's): another backward needs another forward run
         if (first_kept > 0) a->recorded = false;
     }
+    theta_reduce_kernel<<<b->nseg, 256, 0, st>>>(b->d_specs, a->theta_id, a->d_theta);
     cudaEventRecord(a->e1, st);
     if (dpos0) cudaMemcpyAsync(dpos0, a->xbar_id, n * sizeof(float4), cudaMemcpyDeviceToHost, st);
     if (dvel0) cudaMemcpyAsync(dvel0, a->vbar_id, n * sizeof(float4), cudaMemcpyDeviceToHost, st);

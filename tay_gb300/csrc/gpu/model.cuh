@@ -152,7 +152,7 @@ bool launch_see_t(const SeeLaunch &L, size_t smem, cudaStream_t st) {
 }
 template <class A>
 void launch_act_t(const ActLaunch &L, cudaStream_t st) {
-    if (L.tiles) act_kernel<A><<<L.tiles, kSortThreads, 0, st>>>(L);
+    if (L.tiles) act_kernel<A><<<L.tiles * kActBlocks, kSortThreads, 0, st>>>(L);
 }
 template <class P>
 cudaError_t prepare_see_t(size_t smem) {

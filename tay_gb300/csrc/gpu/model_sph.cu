@@ -184,7 +184,7 @@ struct Force {
         if (!(r2 < c.support2 && r2 > 0.0f)) return false;
         float4 bv;
         float brho, bA;
-        if constexpr (std::is_same_v<Acc, see_detail::PackedSeen>) {
+        if constexpr (see_detail::IsPacked<Acc>::value) {
             bv = acc.hi;
             brho = acc.hi.w;
             bA = acc.lo.w;
@@ -301,12 +301,15 @@ const ProgramDesc kPrograms[] = {
 // Streams of the adjoint (a separate PassIO, sorted order of the step being reversed):
 //   f4 [0] POS, [1] VEL, [2] RP = {rho, P}, [3] ABAR (adjoint of the acceleration),
 //   [4] XBAR, [5] VBAR (adjoints of the step's initial position and velocity),
-//   [6] RHOBAR, [7] THETA = {d/dalpha, d/dc0} per particle; u32 [0] GID (global id).
+//   [6] RHOBAR = {x, y, z, adjoint of rho}: with the position beside it, it is all that the
+//   density adjoint reads of a neighbour, [7] THETA = {d/dalpha, d/dc0} per particle;
+//   u32 [0] GID (global id).  A force adjoint that replays a list reads positions, velocities,
+//   rho and A packed as the forward force pass does (slot A_PACK, where it reads no RHOBAR).
 // The force is antisymmetric, f_jk = -f_kj (same |x|, s = v.x and rho_bar for both
 // orders), so every term a particle receives from its neighbours' accelerations is a
 // gather with weight (abar_k - abar_j): the adjoint passes are see passes over the same
 // neighbours as the forward ones.
-enum { A_POS = 0, A_VEL = 1, A_RP = 2, A_ABAR = 3, A_XBAR = 4, A_VBAR = 5, A_RHOBAR = 6, A_THETA = 7 };
+enum { A_POS = 0, A_VEL = 1, A_RP = 2, A_ABAR = 3, A_XBAR = 4, A_VBAR = 5, A_RHOBAR = 6, A_THETA = 7, A_PACK = 6 };
 enum { A_GID = 0 };
 
 // integrate (v' = v + dt (a + g), x' = x + dt v', walls) reversed; the wall test is
@@ -334,6 +337,11 @@ struct IntegrateAdj {
         io.out_f4[A_XBAR][i] = make_float4(ybar[0], ybar[1], ybar[2], 0.0f);
         io.out_f4[A_VBAR][i] = make_float4(ubar[0], ubar[1], ubar[2], 0.0f);
         io.out_f4[A_ABAR][i] = make_float4(abar[0], abar[1], abar[2], 0.0f);
+        if (io.out_f4[A_PACK]) {  // for a force adjoint that replays a list
+            const float4 rp = io.in_f4[A_RP][i];
+            io.out_f4[A_PACK][2 * (size_t)i] = make_float4(x.x, x.y, x.z, rp.z);
+            io.out_f4[A_PACK][2 * (size_t)i + 1] = make_float4(v.x, v.y, v.z, rp.x);
+        }
     }
 };
 
@@ -385,14 +393,49 @@ struct ForceAdj {
         float xwv, d[3];     // vbar's: xwv * d
         float xmD, rb;       // Pbar's xmD; rhobar's xmD * rb
         float ad, al, c0;    // theta's: ad * (al, c0)
+        float one;           // 1, for the sums of a single word (LaneSums)
     };
+    // the seer's ten sums, each of products of two words of the term: x + y rounds as fma(1, x, y)
+    static constexpr int kSums = 10;
+    TGPU_D static uint2 sum_of(int c) {
+        switch (c) {
+            case 0: case 1: case 2: return make_uint2(12, (uint32_t)c);      // xbar += xw
+            case 3: case 4: case 5: return make_uint2(3, (uint32_t)c + 1u);  // vbar += xwv d
+            case 6: return make_uint2(7, 8);                                 // rhobar += xmD rb
+            case 7: return make_uint2(12, 7);                                // Pbar += xmD
+            case 8: return make_uint2(9, 10);                                // theta += ad al
+            default: return make_uint2(9, 11);                               //          ad c0
+        }
+    }
+    TGPU_D static float &sum(Seer &s, int c) {
+        switch (c) {
+            case 0: case 1: case 2: return s.xb[c];
+            case 3: case 4: case 5: return s.vb[c - 3];
+            case 6: return s.rhob;
+            case 7: return s.Pb;
+            case 8: return s.ta;
+            default: return s.tc;
+        }
+    }
     template <class Acc>
     TGPU_D static bool term(const Seer &s, const float4 &a, const float4 &b, const Acc &acc, uint32_t j, const Ctx &c,
                             Term &t) {
         const float dx = a.x - b.x, dy = a.y - b.y, dz = a.z - b.z;
         const float r2 = dist2(dx, dy, dz);
         if (!(r2 < c.support2 && r2 > 0.0f)) return false;
-        const float4 bv = acc.f4(1, j), brp = acc.f4(2, j), bab = acc.f4(3, j);
+        const float4 bab = acc.f4(3, j);
+        float4 bv;
+        float brho, bA;
+        if constexpr (see_detail::IsPacked<Acc>::value) {
+            bv = acc.hi;
+            brho = acc.hi.w;
+            bA = acc.lo.w;
+        } else {
+            const float4 brp = acc.f4(2, j);
+            bv = acc.f4(1, j);
+            brho = brp.x;
+            bA = brp.z;
+        }
         const float rinv = rsqrtf(r2);
         const float r = __fmul_rn(r2, rinv);
         const float q = __fmul_rn(r, c.inv_h);
@@ -404,7 +447,7 @@ struct ForceAdj {
         const float sv = __fmaf_rn(vz, dz, __fmaf_rn(vy, dy, __fmul_rn(vx, dx)));
         float Pi = 0.0f, Pi_s = 0.0f, Pi_r2 = 0.0f, Pi_rb = 0.0f, Pi_al = 0.0f, Pi_c0 = 0.0f;
         if (sv < 0.0f) {
-            const float inv_rb = __fdividef(2.0f, __fadd_rn(s.rho, brp.x));
+            const float inv_rb = __fdividef(2.0f, __fadd_rn(s.rho, brho));
             const float inv_den = __fdividef(1.0f, __fadd_rn(r2, c.eta2));
             const float k0 = __fmul_rn(__fmul_rn(c.h, inv_den), inv_rb);
             Pi_al = __fmul_rn(__fmul_rn(-c.c0, k0), sv);
@@ -414,7 +457,7 @@ struct ForceAdj {
             Pi_r2 = __fmul_rn(-Pi, inv_den);
             Pi_rb = __fmul_rn(-Pi, inv_rb);
         }
-        const float T = __fadd_rn(__fadd_rn(s.A, brp.z), Pi);
+        const float T = __fadd_rn(__fadd_rn(s.A, bA), Pi);
         const float mD = __fmul_rn(-c.m, D);
         const float cc = __fmul_rn(mD, T);
         const float wx = s.ab.x - bab.x, wy = s.ab.y - bab.y, wz = s.ab.z - bab.z;
@@ -435,6 +478,7 @@ struct ForceAdj {
         t.ad = __fmul_rn(__fmaf_rn(s.ab.z, dz, __fmaf_rn(s.ab.y, dy, __fmul_rn(s.ab.x, dx))), mD);
         t.al = Pi_al;
         t.c0 = Pi_c0;
+        t.one = 1.0f;
         return true;
     }
     TGPU_D static void fold(Seer &s, const Term &t, const Ctx &) {
@@ -453,14 +497,14 @@ struct ForceAdj {
         Term t;
         if (term(s, a, b, acc, j, c, t)) fold(s, t, c);
     }
-    TGPU_D static void finish(Seer &s, const float4 &, const PassIO &io, uint32_t i, const Ctx &c, const Ctx &) {
+    TGPU_D static void finish(Seer &s, const float4 &a, const PassIO &io, uint32_t i, const Ctx &c, const Ctx &) {
         s.Pb *= s.inv_rho2;  // dc/dP_k = -m D / rho_k^2
         const float x = s.rho / c.rho0;
         const float x2 = x * x;
         const float x6 = (x2 * x2) * x2;
         s.rhob += s.Pb * (c.B * 7.0f * x6 / c.rho0);
         s.tc += s.Pb * (2.0f * s.P / c.c0);
-        io.out_f4[A_RHOBAR][i] = make_float4(s.rhob, 0.0f, 0.0f, 0.0f);
+        io.out_f4[A_RHOBAR][i] = make_float4(a.x, a.y, a.z, s.rhob);
         const float4 xb = io.in_f4[A_XBAR][i], vb = io.in_f4[A_VBAR][i];
         io.out_f4[A_XBAR][i] = make_float4(xb.x + s.xb[0], xb.y + s.xb[1], xb.z + s.xb[2], 0.0f);
         io.out_f4[A_VBAR][i] = make_float4(vb.x + s.vb[0], vb.y + s.vb[1], vb.z + s.vb[2], 0.0f);
@@ -473,6 +517,7 @@ struct ForceAdj {
 // same list.
 struct ForceAdjReplay : ForceAdj {
     static constexpr int kPairList = 2;
+    static constexpr int kPack = A_PACK;
     TGPU_D static bool replay_ok(const Ctx &mine, const Ctx &rec) { return mine.support2 <= rec.support2; }
 };
 
@@ -486,7 +531,7 @@ struct DensityAdj {
     using SeeCtx = Ctx;
     using ActCtx = Ctx;
     using Seer = DensityAdjSeer;
-    static constexpr int kSeenF4 = 2;
+    static constexpr int kSeenF4 = 1;  // stream 0 is RHOBAR: the position, and rhobar beside it
     // replays the force adjoint's list (same pairs: r2 < support2, r2 > 0)
     static constexpr int kPairList = 2;
     TGPU_D static bool replay_ok(const Ctx &mine, const Ctx &rec) { return mine.support2 <= rec.support2; }
@@ -497,22 +542,22 @@ struct DensityAdj {
         const float r2 = dist2(a.x - b.x, a.y - b.y, a.z - b.z);
         return r2 < c.support2 && r2 > 0.0f;
     }
-    TGPU_D static int seen_stream(int k) { return k == 0 ? A_POS : A_RHOBAR; }
+    TGPU_D static int seen_stream(int) { return A_POS; }
     TGPU_D static void load(Seer &s, const PassIO &io, uint32_t i, const Ctx &, const Ctx &) {
-        s.rhob = io.in_f4[A_RHOBAR][i].x;
+        s.rhob = io.in_f4[A_POS][i].w;
         s.xb[0] = s.xb[1] = s.xb[2] = 0.0f;
     }
     struct __align__(16) Term {
         float g, dx, dy, dz;
     };
     template <class Acc>
-    TGPU_D static bool term(const Seer &s, const float4 &a, const float4 &b, const Acc &acc, uint32_t j, const Ctx &c,
+    TGPU_D static bool term(const Seer &s, const float4 &a, const float4 &b, const Acc &, uint32_t, const Ctx &c,
                             Term &t) {
         const float dx = a.x - b.x, dy = a.y - b.y, dz = a.z - b.z;
         const float r2 = dist2(dx, dy, dz);
         if (!(r2 < c.support2 && r2 > 0.0f)) return false;
         const float rinv = rsqrtf(r2);
-        t.g = (s.rhob + acc.f4(1, j).x) * c.m * kernel_dw(r2 * rinv * c.inv_h, c.sigma, c.inv_h) * rinv;
+        t.g = (s.rhob + b.w) * c.m * kernel_dw(r2 * rinv * c.inv_h, c.sigma, c.inv_h) * rinv;
         t.dx = dx;
         t.dy = dy;
         t.dz = dz;
@@ -534,13 +579,21 @@ struct DensityAdj {
     }
 };
 
-// adjoints of the step's initial state back to id order (the order of the step before)
+// adjoints of the step's initial state back to id order (the order of the step before), and the
+// particle's parameter gradients onto its sums over the steps (double2 per particle in out
+// slot THETA; added up over the particles once, at the end)
 struct ScatterAdj {
     using ActCtx = Ctx;
     TGPU_D static void act(const PassIO &io, uint32_t i, const Ctx &) {
         const uint32_t gid = io.in_u32[A_GID][i];
         io.out_f4[A_XBAR][gid] = io.in_f4[A_XBAR][i];
         io.out_f4[A_VBAR][gid] = io.in_f4[A_VBAR][i];
+        const float4 t = io.in_f4[A_THETA][i];
+        double2 *sum = reinterpret_cast<double2 *>(io.out_f4[A_THETA]) + gid;
+        double2 v = *sum;
+        v.x += (double)t.x;
+        v.y += (double)t.y;
+        *sum = v;
     }
 };
 

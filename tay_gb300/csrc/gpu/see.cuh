@@ -130,14 +130,26 @@ template <class P>
 struct PackOf<P, decltype((void)P::kPack)> {
     static constexpr int value = P::kPack;
 };
-// One neighbour's packed 32 bytes, in one load; lo's x, y, z are its position.
+// One neighbour's packed 32 bytes, in one load (lo's x, y, z are its position); other streams
+// of it as the pass reads them without.
+template <class Acc>
 struct PackedSeen {
     float4 lo, hi;
-    TGPU_D PackedSeen(const float4 *pack, uint32_t j) {
+    const Acc &rest;
+    TGPU_D PackedSeen(const float4 *pack, uint32_t j, const Acc &acc) : rest(acc) {
         asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
             : "=f"(lo.x), "=f"(lo.y), "=f"(lo.z), "=f"(lo.w), "=f"(hi.x), "=f"(hi.y), "=f"(hi.z), "=f"(hi.w)
             : "l"(pack + 2 * (size_t)j));
     }
+    TGPU_D float4 f4(int k, uint32_t j) const { return rest.f4(k, j); }
+};
+template <class Acc>
+struct IsPacked {
+    static constexpr bool value = false;
+};
+template <class Acc>
+struct IsPacked<PackedSeen<Acc>> {
+    static constexpr bool value = true;
 };
 
 // The walk of a pass that records no pair list.
@@ -356,7 +368,7 @@ TGPU_D void list_run(typename P::Seer &s, const float4 &sp, const PairList &pl, 
     // entries j0 and, with `two`, j1
     auto pair = [&](uint32_t j0, uint32_t j1, bool two) {
         if constexpr (PackOf<P>::value >= 0) {
-            const PackedSeen b0(pack, j0), b1(pack, two ? j1 : j0);
+            const PackedSeen<Acc> b0(pack, j0, acc), b1(pack, two ? j1 : j0, acc);
             if (j0 != self) P::see(s, sp, b0.lo, b0, j0, sctx);
             if (two && j1 != self) P::see(s, sp, b1.lo, b1, j1, sctx);
         } else {
@@ -1054,6 +1066,56 @@ struct TermsOf<P, std::void_t<typename P::Term>> {
     static constexpr bool value = true;
 };
 
+// Sums that a pass with many of them (P::kSums) has its seer's lanes fold side by side, lane c
+// the sums c, c + G, ...: each sum is fma(term[u], term[w], sum) over the terms in order, with
+// u and w from P::sum_of(c) (words of the term, one of which may hold 1), and starts at and
+// ends in P::sum(seer, c).  Folded by every lane alike, the force adjoint's ten sums were half
+// of its instructions.
+template <class P, class = void>
+struct SumsOf {
+    static constexpr int value = 0;
+};
+template <class P>
+struct SumsOf<P, decltype((void)P::kSums)> {
+    static constexpr int value = P::kSums;
+};
+
+// A lane's share of its seer's sums.
+template <class P, int G>
+struct LaneSums {
+    static constexpr int kEach = (SumsOf<P>::value + G - 1) / G;
+    float v[kEach > 0 ? kEach : 1];
+    uint32_t u[kEach > 0 ? kEach : 1], w[kEach > 0 ? kEach : 1];  // word offsets into a term
+
+    TGPU_D void start(typename P::Seer &s, uint32_t sub) {
+        if constexpr (kEach > 0) {
+#pragma unroll
+            for (int e = 0; e < kEach; ++e) {
+                const int c = min((int)sub + e * G, SumsOf<P>::value - 1);
+                const uint2 o = P::sum_of(c);
+                u[e] = o.x;
+                w[e] = o.y;
+                v[e] = 0.0f;
+#pragma unroll
+                for (int k = 0; k < SumsOf<P>::value; ++k)
+                    if (k == c) v[e] = P::sum(s, k);
+            }
+        }
+    }
+    TGPU_D void add(const typename P::Term &t) {
+        const float *f = reinterpret_cast<const float *>(&t);
+#pragma unroll
+        for (int e = 0; e < kEach; ++e) v[e] = __fmaf_rn(f[u[e]], f[w[e]], v[e]);
+    }
+    // Every lane of the seer gets all its sums.
+    TGPU_D void finish(typename P::Seer &s) const {
+        if constexpr (kEach > 0) {
+#pragma unroll
+            for (int k = 0; k < SumsOf<P>::value; ++k) P::sum(s, k) = __shfl_sync(0xffffffffu, v[k / G], k % G, G);
+        }
+    }
+};
+
 // Slots of a seer's queue: two chunks add at most 2 G to what the last ones left.
 constexpr int group_slots(int g) { return g > 8 ? 4 * g : 32; }
 
@@ -1070,15 +1132,22 @@ struct Group {
 };
 
 // Folds a seer's first n <= kMost terms, in order (all its lanes hold the same seer and do the
-// same).
-template <class P, int kMost>
-TGPU_D void fold_terms(typename P::Seer &s, const typename P::Term *q, uint32_t n, const typename P::SeeCtx &c) {
+// same, or share its sums).
+template <class P, int kMost, int G>
+TGPU_D void fold_terms(typename P::Seer &s, LaneSums<P, G> &sums, const typename P::Term *q, uint32_t n,
+                       const typename P::SeeCtx &c) {
+    auto one = [&](const typename P::Term &t) {
+        if constexpr (SumsOf<P>::value > 0)
+            sums.add(t);
+        else
+            P::fold(s, t, c);
+    };
     __syncwarp();
     if (__all_sync(0xffffffffu, n == (uint32_t)kMost)) {
 #pragma unroll
-        for (int k = 0; k < kMost; ++k) P::fold(s, q[k], c);
+        for (int k = 0; k < kMost; ++k) one(q[k]);
     } else {
-        for (uint32_t k = 0; k < n; ++k) P::fold(s, q[k], c);
+        for (uint32_t k = 0; k < n; ++k) one(q[k]);
     }
     __syncwarp();
 }
@@ -1086,12 +1155,13 @@ TGPU_D void fold_terms(typename P::Seer &s, const typename P::Term *q, uint32_t 
 // The terms of up to G candidates of a seer, one a lane (those with `take`), folded in lane
 // order; kPacked: read from `pos` as packed neighbours.
 template <class P, int G, bool kPacked = false, class Acc>
-TGPU_D void eval_terms(typename P::Seer &s, const float4 &sp, bool take, uint32_t j, const float4 *pos,
-                       const Acc &acc, typename P::Term *q, const Group<G> &gr, const typename P::SeeCtx &c) {
+TGPU_D void eval_terms(typename P::Seer &s, LaneSums<P, G> &sums, const float4 &sp, bool take, uint32_t j,
+                       const float4 *pos, const Acc &acc, typename P::Term *q, const Group<G> &gr,
+                       const typename P::SeeCtx &c) {
     typename P::Term t;
     if (take) {
         if constexpr (kPacked) {
-            const PackedSeen b(pos, j);
+            const PackedSeen<Acc> b(pos, j, acc);
             take = P::term(s, sp, b.lo, b, j, c, t);
         } else {
             take = P::term(s, sp, __ldg(pos + j), acc, j, c, t);
@@ -1099,7 +1169,7 @@ TGPU_D void eval_terms(typename P::Seer &s, const float4 &sp, bool take, uint32_
     }
     const uint32_t v = gr.votes(take);
     if (take) q[__popc(v & gr.below)] = t;
-    fold_terms<P, G>(s, q, (uint32_t)__popc(v), c);
+    fold_terms<P, G>(s, sums, q, (uint32_t)__popc(v), c);
 }
 
 // The box test without branches, on the difference the pass's own functions compute.
@@ -1188,6 +1258,8 @@ __global__ void __launch_bounds__(kSeeThreads, 8) see_group_kernel(SeeLaunch L) 
     const float4 *pos = L.io.in_f4[0];
     const uint32_t self = (active && L.skip_self) ? i : 0xFFFFFFFFu;
     uint32_t pairs = 0, tested = 0;
+    LaneSums<P, G> sums;
+    sums.start(s, sub);
     Term *terms = &s_terms[grp][0];
     uint32_t *wait = &s_wait[grp][0];
     uint32_t head = 0, queued = 0;  // of the waiting terms or candidates (the same in a seer's lanes)
@@ -1212,10 +1284,10 @@ __global__ void __launch_bounds__(kSeeThreads, 8) see_group_kernel(SeeLaunch L) 
                     const uint32_t f = t + G;
                     const uint32_t next = f < c.x ? __ldg(e + (size_t)(f >> 2) * stride + (f & 3u)) : self;
                     if constexpr (PackOf<P>::value >= 0)
-                        eval_terms<P, G, true>(s, sp, t < c.x && j != self, j, L.io.in_f4[PackOf<P>::value], acc,
+                        eval_terms<P, G, true>(s, sums, sp, t < c.x && j != self, j, L.io.in_f4[PackOf<P>::value], acc,
                                                terms, gr, sctx);
                     else
-                        eval_terms<P, G>(s, sp, t < c.x && j != self, j, pos, acc, terms, gr, sctx);
+                        eval_terms<P, G>(s, sums, sp, t < c.x && j != self, j, pos, acc, terms, gr, sctx);
                     j = next;
                 }
                 if (sub == 0 && active) pairs += c.y + ((!L.skip_self && box_hit(sp, sp, r4)) ? 1u : 0u);
@@ -1319,13 +1391,13 @@ __global__ void __launch_bounds__(kSeeThreads, 8) see_group_kernel(SeeLaunch L) 
                 }
                 if (__any_sync(0xffffffffu, queued > kSlots - U * G)) {
                     if constexpr (kCheap) {
-                        fold_terms<P, kSlots>(s, terms, queued, sctx);
+                        fold_terms<P, kSlots>(s, sums, terms, queued, sctx);
                         queued = 0;
                     } else {
                         __syncwarp();
                         do {
                             const uint32_t m = min(queued, (uint32_t)G);
-                            eval_terms<P, G>(s, sp, sub < m, wait[(head + sub) & (kSlots - 1u)], pos, acc, terms, gr,
+                            eval_terms<P, G>(s, sums, sp, sub < m, wait[(head + sub) & (kSlots - 1u)], pos, acc, terms, gr,
                                              sctx);
                             head += m;
                             queued -= m;
@@ -1349,16 +1421,17 @@ __global__ void __launch_bounds__(kSeeThreads, 8) see_group_kernel(SeeLaunch L) 
         }
     }
     if constexpr (kCheap) {
-        fold_terms<P, kSlots>(s, terms, queued, sctx);
+        fold_terms<P, kSlots>(s, sums, terms, queued, sctx);
     } else {
         __syncwarp();
         while (__any_sync(0xffffffffu, queued > 0u)) {
             const uint32_t m = min(queued, (uint32_t)G);
-            eval_terms<P, G>(s, sp, sub < m, wait[(head + sub) & (kSlots - 1u)], pos, acc, terms, gr, sctx);
+            eval_terms<P, G>(s, sums, sp, sub < m, wait[(head + sub) & (kSlots - 1u)], pos, acc, terms, gr, sctx);
             head += m;
             queued -= m;
         }
     }
+    sums.finish(s);
     if (active && sub == 0) P::finish(s, sp, L.io, i, sctx, actx);
     if (L.pairs) {
         uint32_t w = warp_sum_u(pairs);
@@ -1379,16 +1452,18 @@ __global__ void __launch_bounds__(kSeeThreads, 8) see_group_kernel(SeeLaunch L) 
     }
 }
 
+// One agent per thread, kActBlocks blocks per radix tile: a block per tile left a launch of
+// 20,480 particles on 12 of the SMs, eight agents after one another in each thread
+// (the adjoint's integrate and scatter passes, which gather by id: 12.4 and 11.7 us).
+constexpr uint32_t kActBlocks = kSortTile / kSortThreads;
 template <class A>
 __global__ void __launch_bounds__(kSortThreads) act_kernel(ActLaunch L) {
-    const uint32_t tile = L.tile_offset + blockIdx.x;
+    const uint32_t tile = L.tile_offset + blockIdx.x / kActBlocks;
     const uint32_t seg = L.tile_seg[tile];
     const SegmentSpec S = L.specs[seg];
     const typename A::ActCtx &actx = *reinterpret_cast<const typename A::ActCtx *>(L.ctx + (size_t)seg * L.ctx_stride);
-    const uint32_t t = tile - S.tile_begin;
-    const uint32_t beg = S.begin + t * kSortTile;
-    const uint32_t end = min(beg + (uint32_t)kSortTile, S.begin + S.count);
-    for (uint32_t i = beg + threadIdx.x; i < end; i += kSortThreads) A::act(L.io, i, actx);
+    const uint32_t k = (tile - S.tile_begin) * kSortTile + (blockIdx.x % kActBlocks) * kSortThreads + threadIdx.x;
+    if (k < S.count) A::act(L.io, S.begin + k, actx);
 }
 
 // AoS <-> SoA conversion for push and fetch (replaces the OpenCL path's whole-buffer
