@@ -59,10 +59,10 @@ TGPU_D float kernel_dw(float q, float sigma, float inv_h) {
     return 0.0f;
 }
 
-TGPU_D float dist2(float dx, float dy, float dz) {
-    float r2 = __fmul_rn(dx, dx);
-    r2 = __fadd_rn(r2, __fmul_rn(dy, dy));
-    return __fadd_rn(r2, __fmul_rn(dz, dz));
+// |a - b|^2, each product and sum rounded separately, on the difference b - a that the walk's
+// box test forms (its negative has the same square).
+TGPU_D float dist2(const float4 &a, const float4 &b) {
+    return see_detail::length2(see_detail::seen_minus_seer(a, b));
 }
 
 TGPU_D float kernel_d2w(float q, float sigma, float inv_h) {
@@ -100,9 +100,10 @@ struct Density {
     static constexpr int kPairList = 1;
     // the see body runs only for pairs inside the support (keep), the particle itself included
     static constexpr bool kKeepGate = true;
+    static constexpr bool kSeenMinusSeer = true;
     TGPU_D static int seen_stream(int) { return POS; }
     TGPU_D static bool keep(const float4 &a, const float4 &b, const Ctx &c) {
-        return dist2(a.x - b.x, a.y - b.y, a.z - b.z) < c.support2;
+        return dist2(a, b) < c.support2;
     }
     TGPU_D static void load(Seer &s, const PassIO &, uint32_t, const Ctx &, const Ctx &) { s.rho = 0.0f; }
     struct Term {
@@ -111,7 +112,7 @@ struct Density {
     template <class Acc>
     TGPU_D static bool term(const Seer &, const float4 &a, const float4 &b, const Acc &, uint32_t, const Ctx &c,
                             Term &t) {
-        const float r2 = dist2(a.x - b.x, a.y - b.y, a.z - b.z);
+        const float r2 = dist2(a, b);
         if (!(r2 < c.support2)) return false;
         t.w = kernel_w(__fsqrt_rn(r2) * c.inv_h, c.sigma);
         return true;
@@ -160,9 +161,10 @@ struct Force {
     TGPU_D static bool replay_ok(const Ctx &mine, const Ctx &rec) { return mine.support2 <= rec.support2; }
     // when it walks: the see body runs only for 0 < r2 < support2
     static constexpr bool kKeepGate = true;
+    static constexpr bool kSeenMinusSeer = true;
     static constexpr bool kKeepRejectsSelf = true;
     TGPU_D static bool keep(const float4 &a, const float4 &b, const Ctx &c) {
-        const float r2 = dist2(a.x - b.x, a.y - b.y, a.z - b.z);
+        const float r2 = dist2(a, b);
         return r2 < c.support2 && r2 > 0.0f;
     }
     TGPU_D static int seen_stream(int k) { return k == 0 ? POS : (k == 1 ? VEL : RP); }
@@ -179,8 +181,9 @@ struct Force {
     template <class Acc>
     TGPU_D static bool term(const Seer &s, const float4 &a, const float4 &b, const Acc &acc, uint32_t j, const Ctx &c,
                             Term &t) {
-        const float dx = a.x - b.x, dy = a.y - b.y, dz = a.z - b.z;
-        const float r2 = dist2(dx, dy, dz);
+        const float3 d = see_detail::seen_minus_seer(a, b);
+        const float dx = -d.x, dy = -d.y, dz = -d.z;
+        const float r2 = see_detail::length2(d);
         if (!(r2 < c.support2 && r2 > 0.0f)) return false;
         float4 bv;
         float brho, bA;
@@ -371,8 +374,9 @@ struct ForceAdj {
     // records the step's pairs inside the support for the density adjoint that follows
     static constexpr int kPairList = 1;
     static constexpr bool kKeepGate = true;
+    static constexpr bool kSeenMinusSeer = true;
     TGPU_D static bool keep(const float4 &a, const float4 &b, const Ctx &c) {
-        return dist2(a.x - b.x, a.y - b.y, a.z - b.z) < c.support2;
+        return dist2(a, b) < c.support2;
     }
     TGPU_D static int seen_stream(int k) { return k == 0 ? A_POS : (k == 1 ? A_VEL : (k == 2 ? A_RP : A_ABAR)); }
     TGPU_D static void load(Seer &s, const PassIO &io, uint32_t i, const Ctx &, const Ctx &) {
@@ -420,8 +424,9 @@ struct ForceAdj {
     template <class Acc>
     TGPU_D static bool term(const Seer &s, const float4 &a, const float4 &b, const Acc &acc, uint32_t j, const Ctx &c,
                             Term &t) {
-        const float dx = a.x - b.x, dy = a.y - b.y, dz = a.z - b.z;
-        const float r2 = dist2(dx, dy, dz);
+        const float3 d = see_detail::seen_minus_seer(a, b);
+        const float dx = -d.x, dy = -d.y, dz = -d.z;
+        const float r2 = see_detail::length2(d);
         if (!(r2 < c.support2 && r2 > 0.0f)) return false;
         const float4 bab = acc.f4(3, j);
         float4 bv;
@@ -537,9 +542,10 @@ struct DensityAdj {
     TGPU_D static bool replay_ok(const Ctx &mine, const Ctx &rec) { return mine.support2 <= rec.support2; }
     // when it walks: the see body runs only for 0 < r2 < support2
     static constexpr bool kKeepGate = true;
+    static constexpr bool kSeenMinusSeer = true;
     static constexpr bool kKeepRejectsSelf = true;
     TGPU_D static bool keep(const float4 &a, const float4 &b, const Ctx &c) {
-        const float r2 = dist2(a.x - b.x, a.y - b.y, a.z - b.z);
+        const float r2 = dist2(a, b);
         return r2 < c.support2 && r2 > 0.0f;
     }
     TGPU_D static int seen_stream(int) { return A_POS; }
@@ -553,8 +559,9 @@ struct DensityAdj {
     template <class Acc>
     TGPU_D static bool term(const Seer &s, const float4 &a, const float4 &b, const Acc &, uint32_t, const Ctx &c,
                             Term &t) {
-        const float dx = a.x - b.x, dy = a.y - b.y, dz = a.z - b.z;
-        const float r2 = dist2(dx, dy, dz);
+        const float3 d = see_detail::seen_minus_seer(a, b);
+        const float dx = -d.x, dy = -d.y, dz = -d.z;
+        const float r2 = see_detail::length2(d);
         if (!(r2 < c.support2 && r2 > 0.0f)) return false;
         const float rinv = rsqrtf(r2);
         t.g = (s.rhob + b.w) * c.m * kernel_dw(r2 * rinv * c.inv_h, c.sigma, c.inv_h) * rinv;

@@ -295,12 +295,12 @@ TGPU_D void lane_one(typename P::Seer &s, const float4 &sp, const float4 &b, con
         bool hit;
         if constexpr (SeenMinusSeerOf<P>::value) {
             const float3 d = seen_minus_seer(sp, b);
-            hit = !(fabsf(d.x) > r4.x) && !(fabsf(d.y) > r4.y) && !(fabsf(d.z) > r4.z);
+            hit = (int)!(fabsf(d.x) > r4.x) & (int)!(fabsf(d.y) > r4.y) & (int)!(fabsf(d.z) > r4.z);
         } else {
             hit = !(fabsf(sp.x - b.x) > r4.x) && !(fabsf(sp.y - b.y) > r4.y) && !(fabsf(sp.z - b.z) > r4.z);
         }
         pairs += hit ? 1u : 0u;
-        if (hit && (SelfSafeOf<P>::value || j != self) && P::keep(sp, b, sctx)) {
+        if ((int)hit & (int)(SelfSafeOf<P>::value || j != self) & (int)P::keep(sp, b, sctx)) {
             if constexpr (kRec) record_kept(*rec, j);
             P::see(s, sp, b, acc, j, sctx);
         }
