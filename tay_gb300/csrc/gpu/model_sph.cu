@@ -101,6 +101,7 @@ struct Density {
     // the see body runs only for pairs inside the support (keep), the particle itself included
     static constexpr bool kKeepGate = true;
     static constexpr bool kSeenMinusSeer = true;
+    static constexpr int kLaneUnroll = 3;  // (524,288 particles, density pass: 916 us at 2, 892 at 3, 900 at 4)
     TGPU_D static int seen_stream(int) { return POS; }
     TGPU_D static bool keep(const float4 &a, const float4 &b, const Ctx &c) {
         return dist2(a, b) < c.support2;
