@@ -111,9 +111,11 @@ uint32_t next_pow2(uint32_t v) {
 constexpr float kFill = 32.0f / 27.0f;
 constexpr uint32_t kFillAgents = 16384;
 
-// Largest segment that one launch sorts (a cluster of 8 blocks); larger ones take the
-// general path, which spreads them over more of the chip.
-constexpr uint32_t kClusterAgents = 16384;
+// Largest segment that one launch boxes, keys and sorts, and largest that a cluster sorts with
+// a launch per radix pass (a change of the keys' width is then one launch more or less, as
+// with the general path); beyond, the general path spreads the work over more of the chip.
+constexpr uint32_t kOneLaunchAgents = 16384;
+constexpr uint32_t kClusterAgents = 131072;
 
 uint32_t log2u(uint32_t v) {
     uint32_t n = 0;
@@ -395,11 +397,11 @@ int tgpu::prepare_specs(TgpuBatch *b) {
     for (auto &kv : b->graphs) cudaGraphExecDestroy(kv.second);
     b->graphs.clear();
     // box reset, bounding box (+ grids), keys and histograms (+ digit offsets), one kernel
-    // per radix pass (or one kernel for all of these), cell table (+ reorder), the passes, and the table clear when it is
+    // per radix pass (or one kernel for all of these, or per pass), cell table (+ reorder), the passes, and the table clear when it is
     // a kernel (Morton order, or more segments than separate header memsets)
     const int passes = sort_passes(b->key_bits);
     const bool clear_kernel = b->cell_order != kOrderRows || b->nseg > kMemsetClearSegments;
-    const int sort = b->cluster_blocks ? 1 : 2 + 1 + passes;
+    const int sort = !b->cluster_blocks ? 2 + 1 + passes : b->cluster_split ? passes : 1;
     b->launches_per_step = sort + 1 + (int)b->runs.size() + (clear_kernel ? 1 : 0);
     return TGPU_OK;
 }
@@ -447,6 +449,7 @@ SortLaunch tgpu::sort_launch(TgpuBatch *b) {
     L.key_bits = b->key_bits;
     L.cluster_blocks = b->cluster_blocks;
     L.cluster_items = b->cluster_items;
+    L.cluster_split = b->cluster_split;
     return L;
 }
 
@@ -986,6 +989,7 @@ int alloc_batch(TgpuBatch *b) {
     uint32_t largest = 0;
     for (const auto &sp : b->specs) largest = std::max(largest, sp.count);
     cluster_sort_shape((uint32_t)b->nseg, largest, kClusterAgents, &b->cluster_blocks, &b->cluster_items);
+    b->cluster_split = largest > kOneLaunchAgents ? 1u : 0u;
     return TGPU_OK;
 }
 

@@ -68,7 +68,7 @@ struct TgpuBatch {
     std::vector<uint32_t> cta_begin;           // first CTA of each segment, + total
     std::vector<TgpuStatePass> state_passes;   // tgpu_state_create: the state's pass list
     uint32_t tiles = 0, ctas = 0, key_bits = 0;
-    uint32_t cluster_blocks = 0, cluster_items = 0;  // SortLaunch::cluster_blocks, cluster_items
+    uint32_t cluster_blocks = 0, cluster_items = 0, cluster_split = 0;  // SortLaunch's
     bool specs_dirty = true;
     float fill = 0.0f;  // SegmentSpec::fill of every segment
 

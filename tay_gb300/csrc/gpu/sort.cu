@@ -559,13 +559,17 @@ TGPU_D uint2 block_scan2(uint32_t a, uint32_t b, uint32_t (*sums)[kClusterWarps]
     return make_uint2(sums[0][warp] + ia - a, sums[1][warp] + ib - b);
 }
 
-// gridDim.x = segments * cluster size; block chunks of 1 << chunk_bits agents.
+// gridDim.x = segments * cluster size; block chunks of 1 << chunk_bits agents.  The launch runs
+// the radix passes of the key bits [first_bit, end_bit): from 0, after box, grid and keys;
+// else of the keys and permutation in keys_in / vals_in.
 template <int kItems>
 __global__ void __launch_bounds__(kClusterThreads, 1)
     cluster_sort_kernel(const SegmentSpec *__restrict__ specs, const float4 *__restrict__ pos,
                         const float4 *__restrict__ pos_max, BoxAcc *__restrict__ box, SegGrid *__restrict__ grids,
+                        const uint32_t *__restrict__ keys_in, const uint32_t *__restrict__ vals_in,
                         uint32_t *__restrict__ keys_out, uint32_t *__restrict__ vals_out, uint32_t blocks,
-                        uint32_t key_bits, uint32_t digit_bits, uint32_t chunk_bits) {
+                        uint32_t key_bits, uint32_t digit_bits, uint32_t chunk_bits, uint32_t first_bit,
+                        uint32_t end_bit) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     ClusterSmem<kItems> &sm = *reinterpret_cast<ClusterSmem<kItems> *>(smem_raw);
     const uint32_t seg = blockIdx.x / blocks, rank = cluster_rank();
@@ -578,88 +582,98 @@ __global__ void __launch_bounds__(kClusterThreads, 1)
     // every block of the cluster runs before its shared memory is written (awaited below)
     asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
 
-    // ---- bounding box (bbox_kernel's rules), this block's agents in the order of the ranking
-    float3 p[kItems];
-    uint32_t v[9];
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        v[a] = 0xFFFFFFFFu;
-        v[3 + a] = 0u;
-        v[6 + a] = float_to_ordered(0.0f);
-    }
-#pragma unroll
-    for (int r = 0; r < kItems; ++r) {
-        const uint32_t k = warp * per_warp + r * 32u + lane;
-        if (k >= have) continue;
-        const float4 q = pos[s.begin + begin + k];
-        p[r] = make_float3(q.x, q.y, q.z);
-        const float c[3] = {q.x, q.y, q.z};
-        if (!s.fixed_box)
-            for (int a = 0; a < 3; ++a) {
-                const uint32_t o = float_to_ordered(c[a]);
-                v[a] = min(v[a], o);
-                v[3 + a] = max(v[3 + a], o);
-            }
-        if (pos_max) {
-            const float4 m = pos_max[s.begin + begin + k];
-            const float d[3] = {m.x - q.x, m.y - q.y, m.z - q.z};
-            for (int a = 0; a < 3; ++a) v[6 + a] = max(v[6 + a], float_to_ordered(fmaxf(d[a], 0.0f)));
-        }
-    }
-#pragma unroll
-    for (int a = 0; a < 9; ++a) {
-        const uint32_t w = a < 3 ? __reduce_min_sync(0xffffffffu, v[a]) : __reduce_max_sync(0xffffffffu, v[a]);
-        if (lane == 0) sm.red[a][warp] = w;
-    }
-    __syncthreads();
-    asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
-    if (warp < 9) {
-        const uint32_t x = sm.red[warp][lane];
-        const uint32_t w = warp < 3 ? __reduce_min_sync(0xffffffffu, x) : __reduce_max_sync(0xffffffffu, x);
-        if (lane < blocks) remote_store(remote_addr(&sm.boxes[rank][warp], lane), w);
-    }
-    cluster_barrier();
-    if (warp == 0) {
-        const uint32_t a = lane < 3u ? lane : 2u;
-        uint32_t lo = 0xFFFFFFFFu, hi = 0u, size = 0u;
-        for (uint32_t q = 0; q < blocks; ++q) {
-            lo = min(lo, sm.boxes[q][a]);
-            hi = max(hi, sm.boxes[q][3 + a]);
-            size = max(size, sm.boxes[q][6 + a]);
-        }
-        derive_grid(specs[seg], lo, hi, &sm.grid);
-        if (rank == 0 && lane < 3u) {
-            box[seg].lo[lane] = lo;
-            box[seg].hi[lane] = hi;
-            box[seg].size[lane] = size;
-        }
-        __syncwarp();
-        if (rank == 0 && lane == 0) grids[seg] = sm.grid;
-    }
-    __syncthreads();
-
-    // ---- keys
     uint32_t key[kItems], val[kItems];
-    {
-        const Grid g = sm.grid.g;
+    if (first_bit == 0) {
+        // ---- bounding box (bbox_kernel's rules), this block's agents in the order of the ranking
+        float3 p[kItems];
+        uint32_t v[9];
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            v[a] = 0xFFFFFFFFu;
+            v[3 + a] = 0u;
+            v[6 + a] = float_to_ordered(0.0f);
+        }
 #pragma unroll
         for (int r = 0; r < kItems; ++r) {
             const uint32_t k = warp * per_warp + r * 32u + lane;
-            key[r] = 0u;
-            val[r] = s.begin + begin + k;
             if (k >= have) continue;
-            key[r] = cell_key(s, (uint32_t)cell_coord(p[r].x, g.origin[0], g.inv_cs[0], g.dims[0]),
-                              (uint32_t)cell_coord(p[r].y, g.origin[1], g.inv_cs[1], g.dims[1]),
-                              (uint32_t)cell_coord(p[r].z, g.origin[2], g.inv_cs[2], g.dims[2]));
+            const float4 q = pos[s.begin + begin + k];
+            p[r] = make_float3(q.x, q.y, q.z);
+            const float c[3] = {q.x, q.y, q.z};
+            if (!s.fixed_box)
+                for (int a = 0; a < 3; ++a) {
+                    const uint32_t o = float_to_ordered(c[a]);
+                    v[a] = min(v[a], o);
+                    v[3 + a] = max(v[3 + a], o);
+                }
+            if (pos_max) {
+                const float4 m = pos_max[s.begin + begin + k];
+                const float d[3] = {m.x - q.x, m.y - q.y, m.z - q.z};
+                for (int a = 0; a < 3; ++a) v[6 + a] = max(v[6 + a], float_to_ordered(fmaxf(d[a], 0.0f)));
+            }
         }
+#pragma unroll
+        for (int a = 0; a < 9; ++a) {
+            const uint32_t w = a < 3 ? __reduce_min_sync(0xffffffffu, v[a]) : __reduce_max_sync(0xffffffffu, v[a]);
+            if (lane == 0) sm.red[a][warp] = w;
+        }
+        __syncthreads();
+        asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
+        if (warp < 9) {
+            const uint32_t x = sm.red[warp][lane];
+            const uint32_t w = warp < 3 ? __reduce_min_sync(0xffffffffu, x) : __reduce_max_sync(0xffffffffu, x);
+            if (lane < blocks) remote_store(remote_addr(&sm.boxes[rank][warp], lane), w);
+        }
+        cluster_barrier();
+        if (warp == 0) {
+            const uint32_t a = lane < 3u ? lane : 2u;
+            uint32_t lo = 0xFFFFFFFFu, hi = 0u, size = 0u;
+            for (uint32_t q = 0; q < blocks; ++q) {
+                lo = min(lo, sm.boxes[q][a]);
+                hi = max(hi, sm.boxes[q][3 + a]);
+                size = max(size, sm.boxes[q][6 + a]);
+            }
+            derive_grid(specs[seg], lo, hi, &sm.grid);
+            if (rank == 0 && lane < 3u) {
+                box[seg].lo[lane] = lo;
+                box[seg].hi[lane] = hi;
+                box[seg].size[lane] = size;
+            }
+            __syncwarp();
+            if (rank == 0 && lane == 0) grids[seg] = sm.grid;
+        }
+        __syncthreads();
+
+        // ---- keys
+        {
+            const Grid g = sm.grid.g;
+#pragma unroll
+            for (int r = 0; r < kItems; ++r) {
+                const uint32_t k = warp * per_warp + r * 32u + lane;
+                key[r] = 0u;
+                val[r] = s.begin + begin + k;
+                if (k >= have) continue;
+                key[r] = cell_key(s, (uint32_t)cell_coord(p[r].x, g.origin[0], g.inv_cs[0], g.dims[0]),
+                                  (uint32_t)cell_coord(p[r].y, g.origin[1], g.inv_cs[1], g.dims[1]),
+                                  (uint32_t)cell_coord(p[r].z, g.origin[2], g.inv_cs[2], g.dims[2]));
+            }
+        }
+    } else {
+#pragma unroll
+        for (int r = 0; r < kItems; ++r) {
+            const uint32_t k = warp * per_warp + r * 32u + lane;
+            key[r] = k < have ? keys_in[s.begin + begin + k] : 0u;
+            val[r] = k < have ? vals_in[s.begin + begin + k] : 0u;
+        }
+        asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
     }
 
     // ---- radix passes
     const uint32_t radix = 1u << digit_bits;
-    for (uint32_t shift = 0, pass = 0; shift < key_bits; shift += digit_bits, ++pass) {
+    for (uint32_t shift = first_bit, pass = 0; shift < end_bit; shift += digit_bits, ++pass) {
         uint2 *mine = sm.buf[pass & 1u], *next = sm.buf[(pass & 1u) ^ 1u];
         const uint32_t mask = (1u << min(digit_bits, key_bits - shift)) - 1u;
-        const bool last = shift + digit_bits >= key_bits;
+        const bool last = shift + digit_bits >= end_bit;
         for (uint32_t i = threadIdx.x; i < kClusterWarps * kMaxRadix / 2u; i += kClusterThreads)
             reinterpret_cast<uint32_t *>(&sm.warp_hist[0][0])[i] = 0u;
         if (pass) {
@@ -876,10 +890,11 @@ Scratch scratch_of(const SortLaunch &L) {
 
 namespace {
 
-// The cluster sort, kItems agents a thread: its launch, or its attributes alone (`launch`
-// false).
+// The cluster sort, kItems agents a thread: launched, with the buffers (0 or 1) that hold the
+// result in *out; or (`launch` false) its attributes set, with the clusters the device can
+// hold in *out.
 template <int kItems>
-cudaError_t cluster_sort(const SortLaunch &L, bool launch, cudaStream_t st, int *clusters) {
+cudaError_t cluster_sort(const SortLaunch &L, bool launch, cudaStream_t st, int *out) {
     auto *kernel = cluster_sort_kernel<kItems>;
     cudaLaunchAttribute attr;
     attr.id = cudaLaunchAttributeClusterDimension;
@@ -895,16 +910,28 @@ cudaError_t cluster_sort(const SortLaunch &L, bool launch, cudaStream_t st, int 
     if (!launch) {
         cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(ClusterSmem<kItems>));
         if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-        if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(clusters, kernel, &cfg);
+        if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(out, kernel, &cfg);
         return e;
     }
     uint32_t chunk_bits = 0;
     while ((1u << chunk_bits) < kItems * (uint32_t)kClusterThreads) ++chunk_bits;
-    return cudaLaunchKernelEx(&cfg, kernel, L.specs, L.pos, L.pos_max, L.box, L.grids, L.keys[1], L.vals[1],
-                              L.cluster_blocks, L.key_bits, (uint32_t)sort_digit_bits(L.key_bits), chunk_bits);
+    const uint32_t digit = (uint32_t)sort_digit_bits(L.key_bits);
+    // all passes in one launch, or one launch a pass
+    const uint32_t step = L.cluster_split ? digit : L.key_bits;
+    int in = 0;
+    cudaError_t e = cudaSuccess;
+    for (uint32_t bit = 0; bit < L.key_bits && e == cudaSuccess; bit += step, in ^= 1)
+        e = cudaLaunchKernelEx(&cfg, kernel, L.specs, L.pos, L.pos_max, L.box, L.grids,
+                               const_cast<const uint32_t *>(L.keys[in]), const_cast<const uint32_t *>(L.vals[in]),
+                               L.keys[in ^ 1], L.vals[in ^ 1], L.cluster_blocks, L.key_bits, digit, chunk_bits, bit,
+                               std::min(L.key_bits, bit + step));
+    *out = in;
+    return e;
 }
-cudaError_t cluster_sort(const SortLaunch &L, bool launch, cudaStream_t st, int *clusters) {
-    return L.cluster_items <= 2 ? cluster_sort<2>(L, launch, st, clusters) : cluster_sort<4>(L, launch, st, clusters);
+cudaError_t cluster_sort(const SortLaunch &L, bool launch, cudaStream_t st, int *out) {
+    return L.cluster_items <= 2   ? cluster_sort<2>(L, launch, st, out)
+           : L.cluster_items <= 4 ? cluster_sort<4>(L, launch, st, out)
+                                  : cluster_sort<8>(L, launch, st, out);
 }
 
 }  // namespace
@@ -913,10 +940,11 @@ bool cluster_sort_shape(uint32_t segments, uint32_t largest, uint32_t most_agent
     *blocks = 0;
     *items = 0;
     if (!segments || largest > most_agents) return false;
-    // 2 agents a thread up to 8 blocks (2,048 agents each), then 4
+    // 2 agents a thread (2,048 a block) as long as the blocks last, then 4, then 8
     SortLaunch L{};
     L.segments = segments;
-    L.cluster_items = largest <= 8u * 2u * kClusterThreads ? 2u : 4u;
+    L.cluster_items = 2;
+    while (L.cluster_items < 8u && largest > kClusterMost * L.cluster_items * kClusterThreads) L.cluster_items *= 2;
     L.cluster_blocks = 1;
     while (L.cluster_blocks * L.cluster_items * kClusterThreads < largest) L.cluster_blocks *= 2;
     if (L.cluster_blocks > kClusterMost || segments * L.cluster_blocks > kClusterWave) return false;
@@ -931,9 +959,10 @@ bool cluster_sort_shape(uint32_t segments, uint32_t largest, uint32_t most_agent
 }
 
 void launch_cluster_sort(const SortLaunch &L, cudaStream_t st, uint32_t **sorted_keys, uint32_t **perm) {
-    cluster_sort(L, true, st, nullptr);
-    *sorted_keys = L.keys[1];
-    *perm = L.vals[1];
+    int out = 1;
+    cluster_sort(L, true, st, &out);
+    *sorted_keys = L.keys[out];
+    *perm = L.vals[out];
 }
 
 void launch_box(const SortLaunch &L, cudaStream_t st) {

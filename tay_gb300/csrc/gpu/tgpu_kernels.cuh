@@ -23,7 +23,8 @@ struct SortLaunch {
     uint32_t tiles;
     uint32_t key_bits;
     uint32_t cluster_blocks;   // blocks per segment of the one-launch sort (0: the general path)
-    uint32_t cluster_items;    // agents per thread of it: 2 or 4
+    uint32_t cluster_items;    // agents per thread of it: 2, 4 or 8
+    uint32_t cluster_split;    // 1: a launch per radix pass
 };
 
 struct GatherSet {

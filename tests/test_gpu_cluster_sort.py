@@ -1,5 +1,5 @@
 """GPU: small segments are boxed, keyed and sorted by one launch (a thread-block cluster per
-segment).  The same keys and a stable sort give the same permutation as the general path,
+segment), middle ones by one such launch per radix pass.  The same keys and a stable sort give the same permutation as the general path,
 which a batch of many segments takes, so the same states alone and in such a batch must end
 with the same bytes."""
 import numpy as np
@@ -12,8 +12,9 @@ from tay_gb300 import workloads as W
 pytestmark = pytest.mark.gpu
 
 # one agent, edges of a warp, of a block's threads and of its chunk, of two, four and eight
-# blocks, and the largest segment
-SIZES = [1, 2, 33, 1023, 1025, 2048, 2049, 4096, 4097, 8193, 16383, 16384]
+# blocks, the largest segment of one launch, and on both sides of the sizes at which a block's
+# chunk grows, up to the largest that a cluster sorts pass by pass
+SIZES = [1, 2, 33, 1023, 1025, 2048, 2049, 4096, 4097, 8193, 16384, 16385, 32769, 65536, 65537, 131072]
 
 
 def _state(model, n, k):
@@ -24,7 +25,7 @@ def _state(model, n, k):
         if k % 3 == 1:
             ps.p[n // 2:, :3] = ps.p[0, :3]       # half of the agents in one place
         return M.boids_setup(mb=4), M.records(M.BOIDS_RECORD, ps.p, ps.v)
-    b = W.box_agents(n, seed=80 + k)
+    b = W.box_agents(n, seed=80 + k, side=1000.0 * max(1.0, n / 20000) ** (1 / 3))
     return M.box_setup(mb=4), M.box_records(b.lo, b.hi, b.v)
 
 
