@@ -208,7 +208,7 @@ extern "C" int tgpu_see_noalloc(const float *positions, unsigned n, const float 
     S.stage_cells = 0;
     S.union_factor = 1;
     S.rows = 1;
-    S.lanes = seer_lanes(n, kNoallocMates, 3, false);
+    S.lanes = seer_lanes(n, kNoallocMates, 3, false, false);
     S.pairs = reinterpret_cast<unsigned long long *>(scratch + kOffPairs);
     S.telemetry = nullptr;
     S.io.in_f4[0] = pos_sorted;

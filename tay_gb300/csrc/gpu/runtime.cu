@@ -281,8 +281,8 @@ void set_lanes(TgpuBatch *b) {
             for (int s = 0; s < b->nseg; ++s)
                 mates += expected_mates(b, s, b->hs[s].passes[r.see_pass].radii) * ((double)b->specs[s].count / std::max(b->total, 1u));
         }
-        r.walk_lanes = seer_lanes(seers, mates, dims, false);
-        r.replay_lanes = seer_lanes(seers, mates, dims, true);
+        r.walk_lanes = seer_lanes(seers, mates, dims, b->m->nonpoint != 0, false);
+        r.replay_lanes = seer_lanes(seers, mates, dims, b->m->nonpoint != 0, true);
     }
 }
 
@@ -291,28 +291,32 @@ void set_lanes(TgpuBatch *b) {
 // Lanes per seer of a see pass over `seers` seers (row order).  With one lane per seer a
 // launch takes at least as long as one lane's walk, and needs enough seers to hide the
 // latency of its loads; below that the chip idles and several lanes share a seer's candidates
-// (see_group_kernel, which issues more instructions per candidate).  The longer a walk, the
-// more seers it takes: `mates` is the number of box-test passes a seer can expect from the
-// seen agents' mean density, and the size up to which 8 lanes win grows with about its cube
-// root.  Measured, us at 1 / 8 / 16 / 32 lanes, see pass (step where marked):
-//   SPH density, 512 mates:  2,048 seers 258 / 65 / 35 / 19, 20,480 433 / 129 / 98 / 84,
-//                            81,920 527 / 386 / 346 / 322, 262,144 1140 / 1162 / 1106 / 1062
-//   SPH force, list replay:  2,048 126 / 33 / 23 / 16, 20,480 147 / 57 / 56 / 67,
-//                            81,920 182 / 159 / 179 / 245, 131,072 233 / 264 / 298 / 400
-//   test model, 100 mates:   2,000 43 / 21 / 16 / 12, 12,000 53 / 24 / 26 / 33,
-//                            30,000 58 / 43 / 45 / 65, 50,000 62 / 63 / 71 / 102
-//   the same (step):  50 mates: 10,000 63 / 47 / 47 / 57, 40,000 72 / 70 / 83 / 117
-//                     25 mates: 5,000 53 / 43 / 43 / 48, 20,000 57 / 51 / 59 / 78, 40,000 61 / 65 / 81 / 116
-//                      4 mates: 10,000 49 / 45 / 49 / 59, 20,000 57 / 58 / 67 / 85
-//   two groups on a plane (step), 25 mates: 8,000 + 10,000 94 / 78 / 93 / 127, 16,000 each
-//                     97 / 92 / 122 / 179, 20,000 + 30,000 99 / 115 / 158 / 248
-uint32_t tgpu::seer_lanes(uint64_t seers, double mates, int dims, bool replay) {
-    const double most = 9000.0 * pow(std::max(mates, 1.0), 0.37) * (dims < 3 ? 0.6 : 1.0);
-    if ((double)seers > most) return 1u;
-    if ((double)seers > most / 4.0) return 8u;
+// (see_group_kernel, which issues more instructions per candidate).  The longer the walk and
+// the heavier its terms, the more seers it takes: `mates` is the number of box-test passes a
+// seer can expect from the seen agents' mean density.  Measured, us at 1 / 8 / 16 / 32 lanes
+// (see pass where marked, else the step):
+//   SPH density (see), 512 mates: 5,120 seers 312 / 94 / 50 / 28, 20,480 207 / 86 / 79 / 74,
+//                                 81,920 268 / 258 / 278 / 282, 131,072 298 / 378 / 429 / 449
+//   SPH force, list replay (see): 5,120 115 / 31 / 22 / 23, 20,480 116 / 49 / 51 / 60,
+//                                 81,920 138 / 142 / 166 / 225
+//   SPH backward sweep, 20,480: 9.3 / 5.3 / 4.7 / 5.1 ms
+//   test model, 100 mates:  2,000 37 / 33 / 27 / 25, 5,000 41 / 36 / 30 / 32,
+//                           12,000 45 / 40 / 40 / 47, 20,000 48 / 48 / 49 / 64, 30,000 51 / 60 / 61 / 82
+//   the same, 50 mates:     10,000 36 / 32 / 31 / 41, 20,000 40 / 41 / 47 / 64
+//             25 mates:     5,000 32 / 27 / 27 / 32, 10,000 34 / 31 / 34 / 43, 20,000 36 / 36 / 45 / 63
+//              4 mates:     5,000 31 / 27 / 29 / 34, 10,000 32 / 30 / 33 / 44, 20,000 39 / 43 / 51 / 70
+//   two groups on a plane, 25 mates: 2,000 each 47 / 43 / 39 / 44, 8,000 + 10,000 54 / 53 / 67 / 101,
+//                           16,000 each 56 / 67 / 97 / 152
+//   box agents (two loads a candidate): 5,000 55 / 35 / 32 / 37, 12,345 71 / 43 / 45 / 52,
+//                           25,000 99 / 80 / 76 / 87, 100,000 301 / 551 / 561 / 684
+uint32_t tgpu::seer_lanes(uint64_t seers, double mates, int dims, bool boxes, bool replay) {
+    const double n = (double)seers, plane = dims < 3 ? 0.6 : 1.0;
+    const double most = 15000.0 * std::min(std::max(mates / 100.0, 1.0), 5.3) * plane * (boxes ? 2.0 : 1.0);
+    if (n > most) return 1u;
     // a dense walk keeps 32 lanes busy row by row; a list of the same seer is shorter
-    if (mates >= 200.0 && !replay) return 32u;
-    return (double)seers > most / 16.0 ? 16u : 32u;
+    if (mates >= 200.0 && !replay) return n > most / 3.0 ? 8u : 32u;
+    if (n > 10000.0 * std::min(mates / 50.0, 2.5) * plane) return 8u;
+    return n > 3500.0 * std::min(mates / 50.0, 1.0) * plane ? 16u : 32u;
 }
 
 // Per-segment grid bounds from the pushed agents: each axis gets a power-of-two cell

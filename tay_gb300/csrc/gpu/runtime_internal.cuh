@@ -129,7 +129,7 @@ namespace tgpu {
 
 // Runtime functions the adjoint module reuses.
 int prepare_specs(TgpuBatch *b);
-uint32_t seer_lanes(uint64_t seers, double mates, int dims, bool replay);
+uint32_t seer_lanes(uint64_t seers, double mates, int dims, bool boxes, bool replay);
 void enqueue_step(TgpuBatch *b, const StepEvents *E = nullptr, bool write_through = false);
 // The batch's pair list on a see launch of run r, when r records or replays one.
 void attach_pair_list(const TgpuBatch *b, const KernelRun &r, SeeLaunch &S);
