@@ -103,8 +103,7 @@ struct TgpuAdjoint {
     float4 *abar = nullptr, *rhobar = nullptr, *theta = nullptr;
     double2 *theta_id = nullptr;  // per particle (id order): gradients summed over the steps
     double *d_theta = nullptr;
-    std::vector<void *> allocs;
-    size_t bytes = 0;
+    tgpu::Arena buffers;
     bool recorded = false;
     double fwd_ms = 0.0, bwd_ms = 0.0;
     cudaEvent_t e0 = nullptr, e1 = nullptr;
@@ -113,36 +112,22 @@ struct TgpuAdjoint {
 namespace tgpu {
 namespace {
 
-template <class T>
-int alloc(TgpuAdjoint *a, T **p, size_t count) {
-    void *q = nullptr;
-    cudaError_t e = cudaMalloc(&q, count * sizeof(T));
-    if (e != cudaSuccess) return fail(TGPU_ERR_CUDA, "adjoint: cudaMalloc of %zu bytes failed: %s", count * sizeof(T),
-                                      cudaGetErrorString(e));
-    a->allocs.push_back(q);
-    a->bytes += count * sizeof(T);
-    *p = static_cast<T *>(q);
-    return TGPU_OK;
+void add_record(TgpuAdjoint *a, Record &r) {
+    const size_t n = std::max<uint32_t>(a->b->total, 1);
+    a->buffers.add(&r.pos, n);
+    a->buffers.add(&r.vel, n);
+    a->buffers.add(&r.rp, n);
+    a->buffers.add(&r.acc, n);
+    a->buffers.add(&r.gid, n);
+    a->buffers.add(&r.keys, n);
+    a->buffers.add(&r.box, (size_t)a->b->nseg);
 }
 
-int alloc_record(TgpuAdjoint *a, Record &r) {
+void add_checkpoint(TgpuAdjoint *a, Checkpoint &c) {
     const size_t n = std::max<uint32_t>(a->b->total, 1);
-    int rc = alloc(a, &r.pos, n);
-    if (!rc) rc = alloc(a, &r.vel, n);
-    if (!rc) rc = alloc(a, &r.rp, n);
-    if (!rc) rc = alloc(a, &r.acc, n);
-    if (!rc) rc = alloc(a, &r.gid, n);
-    if (!rc) rc = alloc(a, &r.keys, n);
-    if (!rc) rc = alloc(a, &r.box, (size_t)a->b->nseg);
-    return rc;
-}
-
-int alloc_checkpoint(TgpuAdjoint *a, Checkpoint &c) {
-    const size_t n = std::max<uint32_t>(a->b->total, 1);
-    int rc = alloc(a, &c.pos, n);
-    if (!rc) rc = alloc(a, &c.vel, n);
-    if (!rc) rc = alloc(a, &c.id, n);
-    return rc;
+    a->buffers.add(&c.pos, n);
+    a->buffers.add(&c.vel, n);
+    a->buffers.add(&c.id, n);
 }
 
 void save_checkpoint(TgpuBatch *b, const Checkpoint &c) {
@@ -342,7 +327,6 @@ extern "C" {
 
 void tgpu_adjoint_destroy(TgpuAdjoint *a) {
     if (!a) return;
-    for (void *p : a->allocs) cudaFree(p);
     if (a->e0) cudaEventDestroy(a->e0);
     if (a->e1) cudaEventDestroy(a->e1);
     delete a;
@@ -373,28 +357,32 @@ int tgpu_adjoint_create(TgpuBatch *b, int steps, int checkpoint_every, int keep_
     a->rec.resize(nrec);
     a->cp.resize(ncp);
     const size_t n = std::max<uint32_t>(b->total, 1);
-    for (auto &r : a->rec)
-        if ((rc = alloc_record(a, r))) break;
-    for (auto &c : a->cp)
-        if (!rc && (rc = alloc_checkpoint(a, c))) break;
-    if (!rc) rc = alloc(a, &a->xbar_id, n);
-    if (!rc) rc = alloc(a, &a->vbar_id, n);
-    if (!rc) rc = alloc(a, &a->xbar_s, n);
-    if (!rc) rc = alloc(a, &a->vbar_s, n);
-    if (!rc) rc = alloc(a, &a->abar, n);
-    if (!rc) rc = alloc(a, &a->rhobar, n);
-    if (!rc) rc = alloc(a, &a->theta, n);
-    if (!rc) rc = alloc(a, &a->theta_id, n);
-    if (!rc) rc = alloc(a, &a->d_theta, 2 * (size_t)b->nseg);
+    for (auto &r : a->rec) add_record(a, r);
+    for (auto &c : a->cp) add_checkpoint(a, c);
+    Arena &A = a->buffers;
+    A.add(&a->xbar_id, n);
+    A.add(&a->vbar_id, n);
+    A.add(&a->xbar_s, n);
+    A.add(&a->vbar_s, n);
+    A.add(&a->abar, n);
+    A.add(&a->rhobar, n);
+    A.add(&a->theta, n);
+    A.add(&a->theta_id, n);
+    A.add(&a->d_theta, 2 * (size_t)b->nseg);
     // per-step lists of one segment when the batch pairs its density and force passes
     // through a list (checkpoint mode only: a list per step of the whole rollout would not fit)
-    if (!rc && checkpoint_every > 0 && b->plist_idx && b->runs.size() == 2 && b->runs[0].list_mode == 1u &&
+    if (checkpoint_every > 0 && b->plist_idx && b->runs.size() == 2 && b->runs[0].list_mode == 1u &&
         b->runs[1].list_mode == 2u) {
         a->lists.resize((size_t)checkpoint_every);
         for (auto &l : a->lists) {
-            if ((rc = alloc(a, &l.idx, (size_t)(b->plist_cap / 4u) * n))) break;
-            if ((rc = alloc(a, &l.count, n))) break;
+            A.add(&l.idx, (size_t)(b->plist_cap / 4u) * n);
+            A.add(&l.count, n);
         }
+    }
+    const cudaError_t e = A.allocate();
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        rc = fail(TGPU_ERR_CUDA, "adjoint: cudaMalloc of %zu bytes failed: %s", A.size(), cudaGetErrorString(e));
     }
     if (!rc && (cudaEventCreate(&a->e0) != cudaSuccess || cudaEventCreate(&a->e1) != cudaSuccess))
         rc = fail(TGPU_ERR_CUDA, "adjoint: cudaEventCreate failed");
@@ -494,6 +482,6 @@ int tgpu_adjoint_backward(TgpuAdjoint *a, const float *dl_dpos, const float *dl_
 
 double tgpu_adjoint_forward_ms(const TgpuAdjoint *a) { return a ? a->fwd_ms : 0.0; }
 double tgpu_adjoint_backward_ms(const TgpuAdjoint *a) { return a ? a->bwd_ms : 0.0; }
-unsigned long long tgpu_adjoint_device_bytes(const TgpuAdjoint *a) { return a ? a->bytes : 0ull; }
+unsigned long long tgpu_adjoint_device_bytes(const TgpuAdjoint *a) { return a ? a->buffers.size() : 0ull; }
 
 }  // extern "C"

@@ -130,26 +130,8 @@ namespace {
 void free_batch(TgpuBatch *b) {
     if (!b) return;
     for (auto &kv : b->graphs) cudaGraphExecDestroy(kv.second);
-    cudaFree(b->d_specs);
-    cudaFree(b->d_extent);
-    cudaFree(b->d_tile_seg);
-    cudaFree(b->d_cta);
-    cudaFree(b->d_box);
-    cudaFree(b->d_grids);
-    for (int c = 0; c < kMaxF4; ++c)
-        for (int k = 0; k < 2; ++k) cudaFree(b->f4[c][k]);
-    for (int c = 0; c < kMaxU32; ++c)
-        for (int k = 0; k < 2; ++k) cudaFree(b->u32[c][k]);
-    for (int k = 0; k < 2; ++k) {
-        cudaFree(b->keys[k]);
-        cudaFree(b->vals[k]);
-    }
-    cudaFree(b->sort_scratch);
-    cudaFree(b->d_status);  // also the error word, the pair counter and the telemetry
     cudaFreeHost(b->h_status);
-    cudaFreeHost(b->h_extent);
     cudaFree(b->table);
-    cudaFree(b->d_aos);
     cudaFree(b->plist_idx);
     cudaFree(b->plist_count);
     cudaFree(b->pack);
@@ -955,40 +937,37 @@ int alloc_batch(TgpuBatch *b) {
     CKR(cudaEventCreate(&b->e0));
     CKR(cudaEventCreate(&b->e1));
     const size_t n = std::max<uint32_t>(b->total, 1);
-    CKR(cudaMalloc(&b->d_specs, sizeof(SegmentSpec) * b->nseg));
-    CKR(cudaMalloc(&b->d_extent, sizeof(BoxAcc)));
-    CKR(cudaMalloc(&b->d_tile_seg, sizeof(uint32_t) * std::max<uint32_t>(b->tiles, 1)));
-    CKR(cudaMalloc(&b->d_cta, sizeof(uint2) * std::max<uint32_t>(b->ctas, 1)));
-    CKR(cudaMalloc(&b->d_box, sizeof(BoxAcc) * b->nseg));
-    CKR(cudaMalloc(&b->d_grids, sizeof(SegGrid) * b->nseg));
+    Arena &A = b->buffers;
+    A.add(&b->d_specs, (size_t)b->nseg);
+    A.add(&b->d_extent, 1);
+    A.add(&b->d_tile_seg, std::max<uint32_t>(b->tiles, 1));
+    A.add(&b->d_cta, std::max<uint32_t>(b->ctas, 1));
+    A.add(&b->d_box, (size_t)b->nseg);
+    A.add(&b->d_grids, (size_t)b->nseg);
+    for (int c = 0; c < m->nu32; ++c)
+        for (int k = 0; k < 2; ++k) A.add(&b->u32[c][k], n);
+    for (int k = 0; k < 2; ++k) {
+        A.add(&b->keys[k], n);
+        A.add(&b->vals[k], n);
+    }
+    A.add(&b->sort_scratch, sort_scratch_bytes((uint32_t)b->nseg, std::max<uint32_t>(b->tiles, 1)) / sizeof(uint32_t));
+    A.add(&b->d_aos, (size_t)m->agent_bytes / 4 * n);
+    // from here on zeroed.  Status block: [0] pair counter, [1..8] telemetry, [9] the device
+    // error word (low half)
+    const size_t zero = A.size();
+    A.add(&b->d_status, kStatusWords);
+    for (int c = 0; c < m->nf4; ++c)
+        for (int k = 0; k < (m->role_f4[c] == kState ? 2 : 1); ++k) A.add(&b->f4[c][k], n);
+    CKR(A.allocate());
+    CKR(cudaMemset(static_cast<char *>(A.data()) + zero, 0, A.size() - zero));
     if (b->tiles) CKR(cudaMemcpy(b->d_tile_seg, b->tile_seg.data(), sizeof(uint32_t) * b->tiles, cudaMemcpyHostToDevice));
     if (b->ctas) CKR(cudaMemcpy(b->d_cta, b->cta.data(), sizeof(uint2) * b->ctas, cudaMemcpyHostToDevice));
-    for (int c = 0; c < m->nf4; ++c) {
-        CKR(cudaMalloc(&b->f4[c][0], sizeof(float4) * n));
-        CKR(cudaMemset(b->f4[c][0], 0, sizeof(float4) * n));
-        if (m->role_f4[c] == kState) {
-            CKR(cudaMalloc(&b->f4[c][1], sizeof(float4) * n));
-            CKR(cudaMemset(b->f4[c][1], 0, sizeof(float4) * n));
-        }
-    }
-    for (int c = 0; c < m->nu32; ++c) {
-        CKR(cudaMalloc(&b->u32[c][0], sizeof(uint32_t) * n));
-        CKR(cudaMalloc(&b->u32[c][1], sizeof(uint32_t) * n));
-    }
-    for (int k = 0; k < 2; ++k) {
-        CKR(cudaMalloc(&b->keys[k], sizeof(uint32_t) * n));
-        CKR(cudaMalloc(&b->vals[k], sizeof(uint32_t) * n));
-    }
-    CKR(cudaMalloc(&b->sort_scratch, sort_scratch_bytes((uint32_t)b->nseg, std::max<uint32_t>(b->tiles, 1))));
-    // status block: [0] pair counter, [1..8] telemetry, [9] the device error word (low half)
-    CKR(cudaMalloc(&b->d_status, sizeof(unsigned long long) * kStatusWords));
-    CKR(cudaMemset(b->d_status, 0, sizeof(unsigned long long) * kStatusWords));
-    CKR(cudaMallocHost(&b->h_status, sizeof(unsigned long long) * kStatusWords));
-    CKR(cudaMallocHost(&b->h_extent, sizeof(BoxAcc) * (size_t)std::max(b->nseg, 1)));
+    // the page-locked status and the extents of the groups' last pushes
+    CKR(cudaMallocHost(&b->h_status, sizeof(unsigned long long) * kStatusWords + sizeof(BoxAcc) * (size_t)std::max(b->nseg, 1)));
+    b->h_extent = reinterpret_cast<BoxAcc *>(b->h_status + kStatusWords);
     b->d_pairs = b->d_status;
     b->d_telemetry = b->d_status + 1;
     b->d_err = reinterpret_cast<uint32_t *>(b->d_status + 9);
-    CKR(cudaMalloc(&b->d_aos, (size_t)m->agent_bytes * n));
     b->ctx_stride = (std::max(m->see_ctx_bytes, m->act_ctx_bytes) + 15u) & ~15u;
     uint32_t largest = 0;
     for (const auto &sp : b->specs) largest = std::max(largest, sp.count);

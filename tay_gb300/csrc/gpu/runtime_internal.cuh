@@ -3,6 +3,7 @@
 
 #include <map>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "model.cuh"
@@ -16,6 +17,35 @@ constexpr int kStatusWords = 10;
 
 // Segments up to which a row-order step clears its table with one memset per segment.
 constexpr int kMemsetClearSegments = 4;
+
+// Device buffers of one object in one allocation: add() every buffer, then one allocate(); each
+// starts on a 256-byte boundary.  (An object of a hundred buffers spent milliseconds in
+// cudaMalloc and cudaFree, one call each.)
+class Arena {
+  public:
+    Arena() = default;
+    Arena(const Arena &) = delete;
+    Arena &operator=(const Arena &) = delete;
+    template <class T>
+    void add(T **p, size_t count) {
+        parts.push_back({reinterpret_cast<void **>(p), bytes});
+        bytes += (count * sizeof(T) + 255) & ~(size_t)255;
+    }
+    cudaError_t allocate() {
+        const cudaError_t e = cudaMalloc(&base, bytes ? bytes : 1);
+        if (e != cudaSuccess) return e;
+        for (const auto &p : parts) *p.first = static_cast<char *>(base) + p.second;
+        return cudaSuccess;
+    }
+    size_t size() const { return bytes; }
+    void *data() const { return base; }
+    ~Arena() { cudaFree(base); }
+
+  private:
+    std::vector<std::pair<void **, size_t>> parts;
+    size_t bytes = 0;
+    void *base = nullptr;
+};
 
 struct KernelRun {
     const KernelDesc *k;
@@ -105,6 +135,7 @@ struct TgpuBatch {
     uint32_t plist_cap = 0;
     float4 *pack = nullptr;  // [2 * total] the neighbour data a recording pass packs (KernelDesc::packs)
 
+    tgpu::Arena buffers;  // what alloc_batch allocates on the device
     cudaStream_t st = nullptr;
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     double last_ms = 0.0;
@@ -112,7 +143,7 @@ struct TgpuBatch {
     bool use_graphs = true;
     uint32_t cell_order = kOrderMorton;  // key order and table layout of every segment
     BoxAcc *d_extent = nullptr;          // pushed extent of one group
-    BoxAcc *h_extent = nullptr;          // page-locked, per segment: the extent of its last push
+    BoxAcc *h_extent = nullptr;          // per segment: the extent of its last push (after h_status)
     uint32_t hit_masks = 0;              // see walk: hit masks (row order)
     std::map<uint64_t, cudaGraphExec_t> graphs;
 
