@@ -142,22 +142,24 @@ TGPU_HD uint32_t axis_max(const SegmentSpec &s, int i) {
 }
 
 // Cell edge as a multiple of `part` for a segment that aims at `fill` agents per cell
-// (SegmentSpec::fill): where its agents, spread over its box, would put more than about three
-// times as many into a cell of the part size, the edge shrinks to the cube root of the ratio,
-// down to a quarter.  Part-size cells hold the 27 cells around a seer's; smaller ones follow
-// its box more closely, which pays when the rows of cells are long.  Measured on an SPH fluid
-// (64 particles per cubed support radius; 1.2 per cell make the edge a third of it): density
-// pass of 524,288 particles 2076 us at multiple 1, 1311 at 1/2, 1122 at 0.45, 977 at 0.34,
-// 1022 at 0.3, 1089 at 1/4; the force pass, whose lists come out in an order with more
-// locality, 963, 886, 813, 766, 744, 800.  Below some 16,000 agents the smaller cells only
-// add radix passes (2,048 particles: 53.6 us per step at 1, 61.1 at 0.34).
+// (SegmentSpec::fill): where its agents, spread over its box, would put several times as many
+// into a cell of the part size, the edge shrinks to a half, a third or a quarter (the nearest
+// to the cube root of the ratio).  Part-size cells hold the 27 cells around a seer's; smaller
+// ones follow its box more closely, which pays when the rows of cells are long.  Fractions
+// 1 / k, and a little more against rounding: a box of twice the part size then never touches
+// more than 2 k + 1 cells of an axis.  Measured on an SPH fluid (64 particles per cubed support
+// radius), density pass of 524,288 particles, us: 2076 at 1 (before the walk's later changes),
+// 1227 at 1/2, 1027 at 0.45, 1172 at 0.4, 1012 at 0.36, 803 at 1.004 / 3, 890 at 0.328, 833 at
+// 0.28; the force pass, whose lists come out in an order with more locality, 963 at 1, 638 at
+// 1/2, 619 at 1/3.  Below some 16,000 agents the smaller cells only add radix passes (2,048
+// particles: 53.6 us per step at 1, 61.1 at 0.34).
 TGPU_HD float fill_multiple(float count, const float *ext, const float *part, int dims, float fill) {
     if (!(fill > 0.0f)) return 1.0f;
     float per_cell = count;
     for (int i = 0; i < dims; ++i)
         if (ext[i] > part[i]) per_cell *= part[i] / ext[i];
-    const float m = cbrtf(fill / per_cell);
-    return m > 0.7f || !(m > 0.0f) ? 1.0f : (m < 0.25f ? 0.25f : m);
+    const float k = rintf(cbrtf(per_cell / fill));
+    return k > 1.0f ? 1.004f / (k < 4.0f ? k : 4.0f) : 1.0f;
 }
 
 TGPU_HD int cell_coord(float p, float origin, float inv_cs, int dim) {

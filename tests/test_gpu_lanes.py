@@ -81,20 +81,22 @@ def test_two_groups_read_every_step(gpu):
         assert x.tobytes() == y.tobytes()
 
 
-@pytest.mark.parametrize("shape,box,dims", [
-    ((32, 40, 16), None, 3),                                   # 64 particles per part: a third
-    ((40, 40, 11), ((0, 0, 0), (2.0, 1.5, 0.8)), 3),           # a fixed box, sparse by the mean: no change
-    ((150, 150, 1), None, 2),                                  # a plane
-    ((20000, 1, 1), None, 3),                                  # a line: one cell across
+@pytest.mark.parametrize("shape,dx,box,dims", [
+    ((32, 40, 16), 0.01, None, 3),                             # 64 particles per cubed part: a third
+    ((32, 40, 16), 0.014, None, 3),                            # 23: a half
+    ((32, 40, 16), 0.007, None, 3),                            # 187 (the lists overflow): a quarter
+    ((40, 40, 11), 0.01, ((0, 0, 0), (2.0, 1.5, 0.8)), 3),     # a fixed box, sparse by the mean: no change
+    ((150, 150, 1), 0.01, None, 2),                            # a plane
+    ((20000, 1, 1), 0.01, None, 3),                            # a line: one cell across
 ])
-def test_cells_below_the_part_size(gpu, shape, box, dims):
+def test_cells_below_the_part_size(gpu, shape, dx, box, dims):
     """Dense SPH groups (above 16,384 particles) get cells below the part size.  The neighbour
     sets do not depend on the cells: the pair counts equal those of cells given by a tuning,
-    and the densities agree to the rounding of a sum of about 250 positive float32 terms
-    (each at most 2^-24 off per addition: 250 * 2^-24 = 1.5e-5 at worst)."""
+    and the densities agree to the rounding of a sum of positive float32 terms (2^-24 for each
+    addition at worst; (0.04 / dx)^3 * 4/3 pi terms, and one in two sums each)."""
     import dataclasses
 
-    sph = W.sph_dam(*shape, tank=(300.0, 3.0, 3.0))
+    sph = W.sph_dam(*shape, dx=dx, tank=(300.0, 3.0, 3.0))
     recs = M.records(M.SPH_RECORD, sph.points.p, sph.points.v)
     setup = dataclasses.replace(M.sph_setup(passes=("sph_density", "sph_pressure"), mb=64), dims=dims, fixed_box=box)
     got = []
@@ -112,4 +114,5 @@ def test_cells_below_the_part_size(gpu, shape, box, dims):
             api.set_tuning()
     assert got[0][0] == got[1][0] > 0
     a, b = got[0][1]["rho"], got[1][1]["rho"]
-    assert np.max(np.abs(a - b) / b) < 1.5e-5
+    terms = (0.04 / dx) ** 3 * 4 / 3 * np.pi
+    assert np.max(np.abs(a - b) / b) < 2 * terms * 2.0 ** -24
