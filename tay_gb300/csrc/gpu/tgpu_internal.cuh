@@ -255,10 +255,14 @@ TGPU_HD uint32_t cell_key(const SegmentSpec &s, uint32_t x, uint32_t y, uint32_t
 }
 
 // A segment's grid for one step with its rounding pad, derived once per step from the
-// bounding box (derive_grid) and read by every later kernel of the step.  The pad is the
-// largest rounding error, in cells, of a cell coordinate computed as
-// floor((p - origin) * inv_cs): a few ulps of the largest coordinate magnitude plus the
-// relative error of the multiply on coordinates up to 1024 cells.
+// bounding box (derive_grid) and read by every later kernel of the step.  The pad is a bound
+// of the rounding error, in cells, of a cell coordinate computed as
+// floor((p - origin) * inv_cs) and of a search interval's ends: 16 ulps of the largest
+// coordinate magnitude (p - r, less the origin, and p - origin round by half an ulp each), plus
+// 4 * 2^-23 of the largest cell coordinate (the rounding of inv_cs and of the product: 1.5 *
+// 2^-23).  No wider than that: with cells of the see radius a seer whose interval crosses one
+// more cell border makes its whole warp walk another row of cells on each side, and a pad of
+// 1/512 cell put one in 256 seers there (see pass of 100,000 test agents 42.7 against 34.5 us).
 struct SegGrid {
     Grid g;
     float pad;
@@ -319,9 +323,11 @@ TGPU_D void derive_grid(const SegmentSpec &s, uint32_t box_lo, uint32_t box_hi, 
     }
     const float m = fmaxf(fabsf(mn), fabsf(mx));
     float all = 0.0f, csmin = __shfl_sync(0xffffffffu, cs, 0);
+    int dmax = 1;
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
         all = fmaxf(all, __shfl_sync(0xffffffffu, m, a));
+        dmax = max(dmax, __shfl_sync(0xffffffffu, d, a));
         csmin = fminf(csmin, __shfl_sync(0xffffffffu, cs, a));
     }
     if (lane < 3u) {
@@ -331,8 +337,8 @@ TGPU_D void derive_grid(const SegmentSpec &s, uint32_t box_lo, uint32_t box_hi, 
         out->g.dims[lane] = d;
     }
     if (lane == 0) {
-        const float ulp = all * 1.1920929e-7f;  // 2^-23
-        out->pad = fmaxf(1.0f / 512.0f, 16.0f * ulp / csmin + 1024.0f * 4.0f * 1.1920929e-7f);
+        const float eps = 1.1920929e-7f;  // 2^-23
+        out->pad = 16.0f * (all * eps) / csmin + (float)dmax * 4.0f * eps;
     }
 }
 #endif
