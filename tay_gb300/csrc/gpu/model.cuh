@@ -61,8 +61,8 @@ struct ModelDesc {
     int nkernels;
     const ProgramDesc *programs;
     int nprograms;
-    // AoS -> SoA; the packed positions' extent is reduced into *extent (reset by the caller)
-    void (*pack)(const uint32_t *aos, uint32_t n, const PassIO &io, BoxAcc *extent, cudaStream_t st);
+    // AoS -> SoA; the packed positions' extent goes to the host through *extent (pack_kernel)
+    void (*pack)(const uint32_t *aos, uint32_t n, const PassIO &io, PushExtent *extent, cudaStream_t st);
     void (*unpack)(uint32_t *aos, uint32_t n, const PassIO &io, uint32_t program, cudaStream_t st);
     int nonpoint;  // 1: box agents, float4 stream 0 the min corner (the position), 1 the max
 };
@@ -165,7 +165,7 @@ cudaError_t prepare_see_t(size_t smem) {
     return cudaFuncSetAttribute(see_rows_kernel<P, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
 }
 template <class M>
-void pack_t(const uint32_t *aos, uint32_t n, const PassIO &io, BoxAcc *extent, cudaStream_t st) {
+void pack_t(const uint32_t *aos, uint32_t n, const PassIO &io, PushExtent *extent, cudaStream_t st) {
     if (n) pack_kernel<M><<<(n + 255) / 256, 256, 0, st>>>(aos, n, io, extent);
 }
 template <class M>

@@ -939,7 +939,7 @@ int alloc_batch(TgpuBatch *b) {
     const size_t n = std::max<uint32_t>(b->total, 1);
     Arena &A = b->buffers;
     A.add(&b->d_specs, (size_t)b->nseg);
-    A.add(&b->d_extent, 1);
+    A.add(&b->d_extent, (size_t)b->nseg);
     A.add(&b->d_tile_seg, std::max<uint32_t>(b->tiles, 1));
     A.add(&b->d_cta, std::max<uint32_t>(b->ctas, 1));
     A.add(&b->d_box, (size_t)b->nseg);
@@ -965,6 +965,12 @@ int alloc_batch(TgpuBatch *b) {
     // the page-locked status and the extents of the groups' last pushes
     CKR(cudaMallocHost(&b->h_status, sizeof(unsigned long long) * kStatusWords + sizeof(BoxAcc) * (size_t)std::max(b->nseg, 1)));
     b->h_extent = reinterpret_cast<BoxAcc *>(b->h_status + kStatusWords);
+    std::vector<PushExtent> extents((size_t)b->nseg);
+    for (int s = 0; s < b->nseg; ++s) {
+        extents[s] = PushExtent{{{~0u, ~0u, ~0u}, {0u, 0u, 0u}, {0u, 0u, 0u}}, 0u, nullptr};
+        CKR(cudaHostGetDevicePointer(reinterpret_cast<void **>(&extents[s].host), b->h_extent + s, 0));
+    }
+    CKR(cudaMemcpy(b->d_extent, extents.data(), sizeof(PushExtent) * (size_t)b->nseg, cudaMemcpyHostToDevice));
     b->d_pairs = b->d_status;
     b->d_telemetry = b->d_status + 1;
     b->d_err = reinterpret_cast<uint32_t *>(b->d_status + 9);
@@ -1283,9 +1289,7 @@ int tgpu_batch_push(TgpuBatch *b, int group, const void *host) {
     }
     // the pack also reduces the extent of the pushed positions (it sizes the segment's
     // grid budget) on the device
-    reset_extent(b->d_extent, b->st);
-    b->m->pack(aos, n, io, b->d_extent, b->st);
-    CK(cudaMemcpyAsync(b->h_extent + group, b->d_extent, sizeof(BoxAcc), cudaMemcpyDeviceToHost, b->st));
+    b->m->pack(aos, n, io, b->d_extent + group, b->st);
     CK(cudaGetLastError());
     if (sized) {
         h.extent_pending = true;

@@ -142,7 +142,7 @@ struct TgpuBatch {
     unsigned long long last_pairs = 0;
     bool use_graphs = true;
     uint32_t cell_order = kOrderMorton;  // key order and table layout of every segment
-    BoxAcc *d_extent = nullptr;          // pushed extent of one group
+    PushExtent *d_extent = nullptr;      // per segment: the pushed extent's accumulator
     BoxAcc *h_extent = nullptr;          // per segment: the extent of its last push (after h_status)
     uint32_t hit_masks = 0;              // see walk: hit masks (row order)
     std::map<uint64_t, cudaGraphExec_t> graphs;

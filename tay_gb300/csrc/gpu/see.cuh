@@ -1473,20 +1473,33 @@ template <class M>
 // records are read (pack) or written (unpack) as one contiguous run of words per block:
 // coalesced in device memory, and large requests when `aos` is page-locked host memory
 // the kernel reads or writes in place (no separate copy).
+//
+// The pack also reduces the extent of the packed positions (the grid budget's input): one
+// atomic per block and axis end, and the last block to finish stores the extent to host memory
+// and leaves the accumulator reset, so a push is this one launch.  (With a reset before it and a
+// copy after it, 32 pushes of some 16,000 agents took 25 us each; the link needs 8.)
 __global__ void __launch_bounds__(256) pack_kernel(const uint32_t *__restrict__ aos, uint32_t n, PassIO io,
-                                                   BoxAcc *extent) {
+                                                   PushExtent *extent) {
     constexpr uint32_t W = M::kAgentBytes / 4;
     __shared__ __align__(16) uint32_t sm[256 * W];
+    __shared__ uint32_t red[6][8];
     const uint32_t first = blockIdx.x * 256u;
     const uint32_t cnt = min(256u, n - first);
     const uint32_t *src = aos + (size_t)first * W;
     const uint32_t words = cnt * W;
     uint32_t w0 = 0;
     if ((reinterpret_cast<uintptr_t>(src) & 15u) == 0) {
-        // 16-byte loads for the aligned bulk, words for the tail
+        // 16-byte loads for the aligned bulk, every one of the thread in flight; words for the tail
+        constexpr uint32_t kLoads = (256u * W / 4u + 255u) / 256u;
         const uint4 *s4 = reinterpret_cast<const uint4 *>(src);
         uint4 *d4 = reinterpret_cast<uint4 *>(sm);
-        for (uint32_t v = threadIdx.x; v < words / 4u; v += 256u) d4[v] = s4[v];
+        uint4 v[kLoads];
+#pragma unroll
+        for (uint32_t k = 0; k < kLoads; ++k)
+            if (k * 256u + threadIdx.x < words / 4u) v[k] = s4[k * 256u + threadIdx.x];
+#pragma unroll
+        for (uint32_t k = 0; k < kLoads; ++k)
+            if (k * 256u + threadIdx.x < words / 4u) d4[k * 256u + threadIdx.x] = v[k];
         w0 = words & ~3u;
     }
     for (uint32_t w = w0 + threadIdx.x; w < words; w += 256u) sm[w] = src[w];
@@ -1494,23 +1507,44 @@ __global__ void __launch_bounds__(256) pack_kernel(const uint32_t *__restrict__ 
     const bool live = threadIdx.x < cnt;
     if (live) M::pack(sm + threadIdx.x * W, io, first + threadIdx.x);
     if (!extent) return;
-    // the extent of the packed positions (the grid budget's input), one atomic per warp
-    // and axis; the thread reads back the position it just wrote
+    // (the thread reads back the position it just wrote)
     float4 p = make_float4(0.f, 0.f, 0.f, 0.f);
     if (live) p = io.out_f4[0][first + threadIdx.x];
     const float c[3] = {p.x, p.y, p.z};
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
-        uint32_t l = live ? float_to_ordered(c[a]) : 0xFFFFFFFFu, h = live ? float_to_ordered(c[a]) : 0u;
-        for (int o = 16; o > 0; o >>= 1) {
-            l = min(l, __shfl_xor_sync(0xffffffffu, l, o));
-            h = max(h, __shfl_xor_sync(0xffffffffu, h, o));
-        }
-        if ((threadIdx.x & 31u) == 0 && l <= h) {
-            atomicMin(&extent->lo[a], l);
-            atomicMax(&extent->hi[a], h);
+        const uint32_t o = float_to_ordered(c[a]);
+        const uint32_t l = __reduce_min_sync(0xffffffffu, live ? o : 0xFFFFFFFFu);
+        const uint32_t h = __reduce_max_sync(0xffffffffu, live ? o : 0u);
+        if ((threadIdx.x & 31u) == 0) {
+            red[a][threadIdx.x >> 5] = l;
+            red[3 + a][threadIdx.x >> 5] = h;
         }
     }
+    __syncthreads();
+    if (threadIdx.x >= 32u) return;
+    if (threadIdx.x < 6u) {
+        uint32_t v = red[threadIdx.x][0];
+        for (int w = 1; w < 8; ++w)
+            v = threadIdx.x < 3u ? min(v, red[threadIdx.x][w]) : max(v, red[threadIdx.x][w]);
+        if (threadIdx.x < 3u)
+            atomicMin(&extent->box.lo[threadIdx.x], v);
+        else
+            atomicMax(&extent->box.hi[threadIdx.x - 3u], v);
+        __threadfence();
+    }
+    __syncwarp();
+    uint32_t last = 0;
+    if (threadIdx.x == 0) last = atomicAdd(&extent->done, 1u) == gridDim.x - 1u;
+    if (!__shfl_sync(0xffffffffu, last, 0)) return;
+    __threadfence();
+    if (threadIdx.x < 3u) {
+        extent->host->lo[threadIdx.x] = __ldcg(&extent->box.lo[threadIdx.x]);
+        extent->host->hi[threadIdx.x] = __ldcg(&extent->box.hi[threadIdx.x]);
+        extent->box.lo[threadIdx.x] = 0xFFFFFFFFu;
+        extent->box.hi[threadIdx.x] = 0u;
+    }
+    if (threadIdx.x == 0) extent->done = 0u;
 }
 
 template <class M>

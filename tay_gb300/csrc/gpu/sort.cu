@@ -131,8 +131,7 @@ __global__ void __launch_bounds__(kSortThreads) bbox_kernel(const SegmentSpec *_
     }
 }
 
-// Resets the box accumulators (and, with `done`, the bbox kernel's block counters); a
-// segment without agents gets its grid here, from the reset box, since no bbox block
+// Resets the box accumulators and the bbox kernel's block counters; a segment without agents gets its grid here, from the reset box, since no bbox block
 // runs for it.  One warp per segment.
 __global__ void box_reset_kernel(BoxAcc *box, uint32_t segments, const SegmentSpec *__restrict__ specs,
                                  SegGrid *__restrict__ grids, uint32_t *done) {
@@ -143,10 +142,8 @@ __global__ void box_reset_kernel(BoxAcc *box, uint32_t segments, const SegmentSp
         box[s].hi[lane_id()] = 0u;
         box[s].size[lane_id()] = float_to_ordered(0.0f);
     }
-    if (done) {
-        if (lane_id() == 0) done[s] = 0u;
-        if (specs[s].tile_count == 0) derive_grid(specs[s], 0xFFFFFFFFu, 0u, grids + s);
-    }
+    if (lane_id() == 0) done[s] = 0u;
+    if (specs[s].tile_count == 0) derive_grid(specs[s], 0xFFFFFFFFu, 0u, grids + s);
 }
 
 // Each segment's grid from its box as it stands (restored boxes of recorded steps): one
@@ -862,10 +859,6 @@ __global__ void __launch_bounds__(kSortThreads) cell_table_kernel(const SegmentS
 }
 
 // ------------------------------------------------------------------ host-side launchers
-
-void reset_extent(BoxAcc *out, cudaStream_t st) {
-    box_reset_kernel<<<1, 32, 0, st>>>(out, 1, nullptr, nullptr, nullptr);
-}
 
 namespace {
 

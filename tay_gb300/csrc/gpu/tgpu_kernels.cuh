@@ -101,6 +101,15 @@ struct SeeLaunch {
     uint32_t lanes;  // row order: lanes per seer (1, 8, 16 or 32; see_group_kernel above 1)
 };
 
+// Extent of a group's pushed positions: accumulated by the pack kernel, stored to page-locked
+// host memory by its last block, which also leaves the accumulator as initialised (lo all
+// ones, hi and done zero).
+struct PushExtent {
+    BoxAcc box;
+    uint32_t done;  // blocks finished
+    BoxAcc *host;   // device address of the host's copy
+};
+
 struct ActLaunch {
     const SegmentSpec *specs;
     const uint32_t *tile_seg;
@@ -134,9 +143,6 @@ constexpr size_t sort_scratch_bytes(uint32_t segments, uint32_t tiles) {
                                (size_t)kMaxSortPasses * tiles * kMaxRadix);
 }
 
-// Bounding box of n positions into *out (reset first), for the pushed extent.
-// Resets an extent accumulator (the pack kernel reduces the pushed positions into it).
-void reset_extent(BoxAcc *out, cudaStream_t st);
 void launch_sort(const SortLaunch &L, cudaStream_t st, uint32_t **sorted_keys, uint32_t **perm);
 // Boxes, grids, keys and sort of small segments in one launch (cluster_sort_kernel), in place
 // of launch_box and launch_sort.  cluster_sort_shape: whether it takes `segments` segments of
