@@ -1055,6 +1055,15 @@ __global__ void __launch_bounds__(kSeeThreads, kStage ? 1 : 8) see_rows_kernel(S
 
 namespace see_detail {
 
+// CTAs per SM that the kernel with several lanes per seer keeps registers for.  Passes with
+// pair lists run many dense seers and want the warps (20,480 SPH particles: step 140 us at 8, 147
+// at 6 or 10); the others the registers (12,345 boxes 41.7 us at 6, 43.0 at 8, 47.5 at 10;
+// four dense flocks of 7,000 agents 57, 61, 62).
+template <class P>
+constexpr int group_ctas() {
+    return ListOf<P>::value ? 8 : 6;
+}
+
 // Whether pass P splits its see function into a term that depends on the pair alone and a
 // fold that adds it to the seer (P::Term, P::term, P::fold).
 template <class P, class = void>
@@ -1200,7 +1209,7 @@ TGPU_D bool box_hit_flat(const float4 &a, const float4 &b, const float4 &r) {
 // seer the same few instructions per neighbour, so more lanes than the chip needs lose (the
 // sizes are at seer_lanes, runtime.cu).
 template <class P, int G, bool kWrite = false>
-__global__ void __launch_bounds__(kSeeThreads, 8) see_group_kernel(SeeLaunch L) {
+__global__ void __launch_bounds__(kSeeThreads, see_detail::group_ctas<P>()) see_group_kernel(SeeLaunch L) {
     using namespace see_detail;
     using Term = typename P::Term;
     constexpr uint32_t kSeers = kSeeThreads / G;
