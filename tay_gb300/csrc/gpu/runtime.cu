@@ -280,7 +280,7 @@ void set_lanes(TgpuBatch *b) {
 //   SPH density (see), 512 mates: 5,120 seers 312 / 94 / 50 / 28, 20,480 207 / 86 / 79 / 74,
 //                                 81,920 268 / 258 / 278 / 282, 131,072 298 / 378 / 429 / 449
 //   SPH force, list replay (see): 5,120 115 / 31 / 22 / 23, 20,480 116 / 49 / 51 / 60,
-//                                 81,920 138 / 142 / 166 / 225
+//                                 81,920 119 / 142 / 166 / 225
 //   SPH backward sweep, 20,480: 9.3 / 5.3 / 4.7 / 5.1 ms
 //   test model, 100 mates:  2,000 37 / 33 / 27 / 25, 5,000 41 / 36 / 30 / 32,
 //                           12,000 45 / 40 / 40 / 47, 20,000 48 / 48 / 49 / 64, 30,000 51 / 60 / 61 / 82

@@ -360,27 +360,38 @@ TGPU_D void lane_run(typename P::Seer &s, const float4 &sp, const float4 &r4, ui
 // recorded order, one group of four per load, two neighbours loaded ahead; words past the
 // n-th are never used; the seer itself is skipped when the pass skips self.  `pack`: the
 // neighbours' packed data of a pass with P::kPack.
+// What bounds it is latency: a group's entries come from HBM (4 bytes a pair, read once), and
+// its neighbours' loads wait for them.  So the next group's entries are loaded before this
+// one's terms, and a pass whose see function rejects the seer itself (kKeepRejectsSelf) has no
+// branch but that test in a pair.  Force pass of 524,288 SPH particles 614 -> 526 us, of 131,072
+// 160 -> 149.  Two groups ahead take registers the terms need (546); four neighbours in flight
+// spill at 8 CTAs per SM (696) and want the warps at 7 or 6 (563, 561).
 template <class P, class Acc>
 TGPU_D void list_run(typename P::Seer &s, const float4 &sp, const PairList &pl, uint32_t i, uint32_t n, uint32_t self,
                      const float4 *pos, const Acc &acc, const float4 *pack, const typename P::SeeCtx &sctx) {
     const uint4 *e = pl.idx + i;
     const size_t stride = pl.stride;
-    // entries j0 and, with `two`, j1
+    constexpr bool kSafe = SelfSafeOf<P>::value;
+    // entries j0 and, with `two`, j1; where the see function does nothing for the seer itself,
+    // the seer stands for an entry past the n-th, so neither needs a branch
     auto pair = [&](uint32_t j0, uint32_t j1, bool two) {
+        if (kSafe && !two) j1 = i;
         if constexpr (PackOf<P>::value >= 0) {
-            const PackedSeen<Acc> b0(pack, j0, acc), b1(pack, two ? j1 : j0, acc);
-            if (j0 != self) P::see(s, sp, b0.lo, b0, j0, sctx);
-            if (two && j1 != self) P::see(s, sp, b1.lo, b1, j1, sctx);
+            const PackedSeen<Acc> b0(pack, j0, acc), b1(pack, two || kSafe ? j1 : j0, acc);
+            if (kSafe || j0 != self) P::see(s, sp, b0.lo, b0, j0, sctx);
+            if (kSafe || (two && j1 != self)) P::see(s, sp, b1.lo, b1, j1, sctx);
         } else {
             const float4 b0 = __ldg(pos + j0);
-            const float4 b1 = two ? __ldg(pos + j1) : b0;
-            if (j0 != self) P::see(s, sp, b0, acc, j0, sctx);
-            if (two && j1 != self) P::see(s, sp, b1, acc, j1, sctx);
+            const float4 b1 = two || kSafe ? __ldg(pos + j1) : b0;
+            if (kSafe || j0 != self) P::see(s, sp, b0, acc, j0, sctx);
+            if (kSafe || (two && j1 != self)) P::see(s, sp, b1, acc, j1, sctx);
         }
     };
+    uint4 next = n ? __ldg(e) : make_uint4(0u, 0u, 0u, 0u);
     for (uint32_t t = 0; t < n; t += 4) {
-        const uint4 g = __ldg(e + (size_t)(t >> 2) * stride);
+        const uint4 g = next;
         const uint32_t m = n - t;  // entries of this group: min(m, 4)
+        if (m > 4u) next = __ldg(e + (size_t)((t >> 2) + 1u) * stride);
         pair(g.x, g.y, m > 1u);
         if (m > 2u) pair(g.z, g.w, m > 3u);
     }

@@ -116,3 +116,31 @@ def test_cells_below_the_part_size(gpu, shape, dx, box, dims):
     a, b = got[0][1]["rho"], got[1][1]["rho"]
     terms = (0.04 / dx) ** 3 * 4 / 3 * np.pi
     assert np.max(np.abs(a - b) / b) < 2 * terms * 2.0 ** -24
+
+
+@pytest.mark.parametrize("most", [2, 9])
+def test_replay_of_short_lists(gpu, most):
+    """Clumps of 1 to `most` particles, further apart than the support: the force pass's lists
+    end at every place of a group of four entries, and the next group's entries are loaded
+    ahead.  One lane per seer (above 16,384 particles), the walk's bits."""
+    k = 1 + np.arange(16384 * 2 // (most + 1) + most) % most
+    site = np.repeat(np.arange(len(k)), k)
+    p = np.zeros((len(site), 4), np.float32)
+    p[:, :3] = 0.1 * np.stack([site % 32, site // 32 % 32, site // 1024], 1) + 0.05
+    p[:, :3] += np.random.default_rng(most).uniform(-0.005, 0.005, (len(site), 3)).astype(np.float32)
+    recs = M.records(M.SPH_RECORD, p, np.zeros_like(p))
+    assert len(recs) > 16384
+    got = []
+    for tuning in ({}, {"pair_list_cap": 0}):
+        api.set_tuning(**tuning)
+        try:
+            b = api.Batch([(M.sph_setup(tank_max=(4.0, 4.0, 4.0), mb=64), recs)])
+            try:
+                b.push()
+                got.append((b.run(1)[1], b.run(1)[1], b.fetch(0).tobytes(), b.telemetry()["replay_warps"]))
+            finally:
+                b.close()
+        finally:
+            api.set_tuning()
+    assert got[0][:3] == got[1][:3]
+    assert got[0][3] == (len(recs) + 127) // 128 * 4 and got[1][3] == 0  # every warp of every block
