@@ -161,18 +161,28 @@ struct NoRec {};
 // to its word of its group of four (measured faster than staging the group in shared
 // memory and storing it whole); a partial last group's other words are never read.
 struct ListRec {
-    uint4 *idx;
-    uint32_t stride, cap, seer, n, other;
+    uint32_t cap, seer, n, other;
+    uint32_t *slot;  // the next entry's word
+    ptrdiff_t wrap;  // words from a group's last entry to the next group's first
+    TGPU_D ListRec(const PairList &l, uint32_t i)
+        : cap(l.cap), seer(i), n(0), other(0), slot(reinterpret_cast<uint32_t *>(l.idx + i)),
+          wrap((ptrdiff_t)l.stride * 4 - 3) {}
 };
+
+// A kept candidate into the recorder's list (the gated walk counts box-test passes itself).  The
+// word's address is stepped, not computed from n: a density walk is bound by issue, and its
+// body runs for some lane at nearly every candidate (524,288 SPH particles, density pass 769 ->
+// 746 us, 131,072 237 -> 225).
+TGPU_D void record_kept(ListRec &r, uint32_t j) {
+    if (r.n < r.cap) *r.slot = j;
+    ++r.n;
+    r.slot += r.n & 3u ? (ptrdiff_t)1 : r.wrap;
+}
 
 template <class P>
 TGPU_D void record_pair(ListRec &r, const float4 &a, const float4 &b, uint32_t j, const typename P::SeeCtx &c) {
     r.other += j != r.seer ? 1u : 0u;
-    if (P::keep(a, b, c)) {
-        if (r.n < r.cap)
-            reinterpret_cast<uint32_t *>(r.idx)[((size_t)(r.n >> 2) * r.stride + r.seer) * 4u + (r.n & 3u)] = j;
-        ++r.n;
-    }
+    if (P::keep(a, b, c)) record_kept(r, j);
 }
 
 // Union walk over candidates [j0, j1) of `src`: batches of up to 32, a box-test phase
@@ -275,12 +285,6 @@ TGPU_D float3 seen_minus_seer(const float4 &a, const float4 &b) {
 TGPU_D float length2(const float3 &d) {
     const float2 m = __fmul2_rn(make_float2(d.x, d.y), make_float2(d.x, d.y));
     return __fadd_rn(__fadd_rn(m.x, m.y), __fmul_rn(d.z, d.z));
-}
-
-// A kept candidate into the recorder's list (the gated walk counts box-test passes itself).
-TGPU_D void record_kept(ListRec &r, uint32_t j) {
-    if (r.n < r.cap) reinterpret_cast<uint32_t *>(r.idx)[((size_t)(r.n >> 2) * r.stride + r.seer) * 4u + (r.n & 3u)] = j;
-    ++r.n;
 }
 
 // One candidate of a lane's walk: the reference's box test and self skip, the pair
@@ -990,7 +994,7 @@ __global__ void __launch_bounds__(kSeeThreads, kStage ? 1 : 8) see_rows_kernel(S
                 // the per-lane walk with the recorder (a block of its own: folded into the
                 // plain walks it costs the non-recording kernels registers)
                 if (active) {
-                    ListRec rec{L.plist.idx, L.plist.stride, L.plist.cap, i, 0u, 0u};
+                    ListRec rec(L.plist, i);
                     const uint32_t before = pairs;
                     for (int z = lo[2]; z <= hi[2]; ++z)
                         for (int y = lo[1]; y <= hi[1]; ++y) {
