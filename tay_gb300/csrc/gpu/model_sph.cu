@@ -97,7 +97,10 @@ struct Density {
     // the see body runs only for pairs inside the support (keep), the particle itself included
     static constexpr bool kKeepGate = true;
     static constexpr bool kSeenMinusSeer = true;
-    static constexpr int kLaneUnroll = 3;  // (524,288 particles, density pass: 916 us at 2, 892 at 3, 900 at 4)
+    // Rows of default cells (a quarter of the support) hold some 9 candidates of a fluid with the
+    // spacing a quarter of its support, and up to 4 left over load together (524,288 particles,
+    // density pass: 687 us at 3, 682 at 4, 619 at 5, 730 at 6; with a third 758, 741, 746 at 3, 4, 5)
+    static constexpr int kLaneUnroll = 5;
     TGPU_D static int seen_stream(int) { return POS; }
     TGPU_D static bool keep(const float4 &a, const float4 &b, const Ctx &c) {
         return dist2(a, b) < c.support2;

@@ -106,10 +106,15 @@ uint32_t next_pow2(uint32_t v) {
     return p;
 }
 
-// Agents per cell that programs with a recording pass aim at, and the agents of a batch from
-// which they do (fill_multiple).
-constexpr float kFill = 32.0f / 27.0f;
-constexpr uint32_t kFillAgents = 16384;
+// Agents per cell (with the default x cells of half the edge) that programs with a recording pass
+// aim at, and the agents of a batch from which they do (fill_multiple); fewer from kFineAgents on,
+// about where such programs go over to one lane per seer.  With the default rule's neighbours for
+// 64 agents per cubed part, us per step at a third / a quarter of the part size: 20,480 agents
+// 138 / 145, 40,960 229 / 236, 81,920 333 / 309, 131,072 415 / 372, 524,288 1299 / 1133.  Less dense
+// groups of 262,144 (1 / 2, 1 / 3, 1 / 4): 32 per cubed part 467, 446, 475; 21 316, 319, 347;
+// 15.6 288, 299, 325.
+constexpr float kFill = 32.0f / 27.0f, kFineFill = 0.72f;
+constexpr uint32_t kFillAgents = 16384, kFineAgents = 80000;
 
 // Largest segment that one launch boxes, keys and sorts, and largest that a cluster sorts with
 // a launch per radix pass (a change of the keys' width is then one launch more or less, as
@@ -1141,7 +1146,8 @@ int tgpu_batch_create(const TgpuGroup *groups, int group_count, TgpuBatch **out)
         g_tuning.cell_multiple != standard.cell_multiple || g_tuning.x_cell_factor != standard.x_cell_factor;
     bool records = false;
     for (int k = 0; k < pd.kernels; ++k) records = records || m->kernels[pd.kernel_index[k]].pair_list == 1;
-    if (records && !own_cells && b->cell_order == kOrderRows && b->total > kFillAgents) b->fill = kFill;
+    if (records && !own_cells && b->cell_order == kOrderRows && b->total > kFillAgents)
+        b->fill = b->total > kFineAgents ? kFineFill : kFill;
     int cursor = 0;
     for (int k = 0; k < pd.kernels && !rc; ++k) {
         KernelRun r{};

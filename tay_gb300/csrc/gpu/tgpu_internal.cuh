@@ -150,9 +150,10 @@ TGPU_HD uint32_t axis_max(const SegmentSpec &s, int i) {
 // more than 2 k + 1 cells of an axis.  Measured on an SPH fluid (64 particles per cubed support
 // radius), density pass of 524,288 particles, us: 2076 at 1 (before the walk's later changes),
 // 1227 at 1/2, 1027 at 0.45, 1172 at 0.4, 1012 at 0.36, 803 at 1.004 / 3, 890 at 0.328, 833 at
-// 0.28; the force pass, whose lists come out in an order with more locality, 963 at 1, 638 at
-// 1/2, 619 at 1/3.  Below some 16,000 agents the smaller cells only add radix passes (2,048
-// particles: 53.6 us per step at 1, 61.1 at 0.34).
+// 0.28; with the walk as it is 878 at 1/2, 746 at 1/3, 619 at 1/4, 713 at 1/5.  The force pass,
+// whose lists come out in an order with more locality, 963 at 1, 638 at 1/2, 619 at 1/3; now 525 at
+// 1/2, 491 at 1/3, 447 at 1/4.  Below some 16,000 agents the smaller cells only add radix passes
+// (2,048 particles: 53.6 us per step at 1, 61.1 at 0.34).
 TGPU_HD float fill_multiple(float count, const float *ext, const float *part, int dims, float fill) {
     if (!(fill > 0.0f)) return 1.0f;
     float per_cell = count;

@@ -85,6 +85,8 @@ def test_two_groups_read_every_step(gpu):
     ((32, 40, 16), 0.01, None, 3),                             # 64 particles per cubed part: a third
     ((32, 40, 16), 0.014, None, 3),                            # 23: a half
     ((32, 40, 16), 0.007, None, 3),                            # 187 (the lists overflow): a quarter
+    ((32, 40, 64), 0.01, None, 3),                             # 64, and above 80,000 particles: a quarter
+    ((44, 44, 44), 0.0126, None, 3),                           # 32: a third
     ((40, 40, 11), 0.01, ((0, 0, 0), (2.0, 1.5, 0.8)), 3),     # a fixed box, sparse by the mean: no change
     ((150, 150, 1), 0.01, None, 2),                            # a plane
     ((20000, 1, 1), 0.01, None, 3),                            # a line: one cell across
