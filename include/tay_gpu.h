@@ -171,7 +171,11 @@ int tgpu_batch_program(const TgpuBatch *batch);
  *                  are read through the L1 cache (more CTAs per SM)
  *   stage_cap      agents staged per CTA (0 = default)
  *   stage_cells    halo cells per CTA (0 = default)
- *   cell_multiple  grid cell edge = cell_multiple x min_part_sizes (0 = 1)
+ *   cell_multiple  grid cell edge = cell_multiple x min_part_sizes (0 = 1).  With the
+ *                  defaults of cell_multiple (1) and x_cell_factor (1/2), batches of more
+ *                  than 16,384 agents whose program records pair lists (SPH) get cells of
+ *                  1/2 to 1/4 of min_part_sizes where the agents are dense; any other pair
+ *                  of values, and a rollout with gradients, uses the cells given
  *   union_factor   a warp walks the union of its seers' cell boxes (one read serves all
  *                  32 lanes) when that union is at most union_factor times the largest
  *                  single box; otherwise each lane walks its own box.  1 (the default; 0
@@ -250,7 +254,7 @@ unsigned long long tgpu_batch_device_bytes(const TgpuBatch *batch);
  * are already in device memory, and writes one float4 per agent to the device buffer
  * `out`, in the input order: x, y, z = the sum, w = the count as int bits.  radii and
  * min_part_sizes are 4 host floats each.  All intermediate buffers live in one fixed
- * array (about 5 MB) of the library's own device memory, which every GPU that loads the
+ * array (about 4 MB) of the library's own device memory, which every GPU that loads the
  * library holds until the process exits; no device memory is allocated.
  *   - n must not exceed tgpu_noalloc_max_agents() (65536); larger calls fail with
  *     TGPU_ERR_ARG and a message from tgpu_noalloc_last_error();
@@ -259,8 +263,8 @@ unsigned long long tgpu_batch_device_bytes(const TgpuBatch *batch);
  *   - every call looks up the array's device address in the current device's context
  *     (a host-side query), so it stays valid after that context is recreated;
  *   - work is enqueued on `stream` (a cudaStream_t, NULL for the default stream) and the
- *     call returns once it has finished: it synchronises and reads back a status word,
- *     so it may not be called while any stream is capturing;
+ *     call returns once it has finished: it synchronises, so it may not be called while
+ *     any stream is capturing;
  *   - a CUDA error pending from earlier work is left in place for its owner and the call
  *     returns TGPU_ERR_CUDA without starting. */
 int tgpu_see_noalloc(const float *positions, unsigned n, const float *radii, const float *min_part_sizes,

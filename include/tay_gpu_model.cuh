@@ -20,6 +20,10 @@
  *     load (the seer's state before its walk), see (one seen agent that passed the box
  *     test; may run on any of the library's walks, so it must not depend on the visiting
  *     order beyond float rounding), finish (the seer's results, plus a fused act);
+ *   - optionally the see function in two parts, P::Term with term (what a pair adds, from
+ *     the pair alone) and fold (adding it): launches of few agents then give a seer several
+ *     lanes, which compute terms side by side and fold them in the walk's order (the same
+ *     bits as see, which must do the same operations);
  *   - per standalone act kernel a policy A with ActCtx and act;
  *   - tgpu::KernelDesc entries (launch_see_t<P> / launch_act_t<A>, prepare_see_t<P>) and
  *     tgpu::ProgramDesc entries (the pass sequences the model runs), gathered in a

@@ -1,7 +1,6 @@
 // Allocation-free neighbour pass: the Z-grid see pass of the test model ("agent_see")
 // run on positions already in device memory, with every intermediate buffer (keys,
-// permutation, radix counts, cell table, reordered positions, accumulators) carved out
-// of one fixed array in the library's own device memory instead of cudaMalloc.
+// permutation, radix counts, cell table, reordered positions) carved out of one fixed array in the library's own device memory instead of cudaMalloc.
 //
 // For callers that cannot allocate device memory at the point where they need the pass:
 // hosts whose memory manager owns the whole device heap (a framework's caching allocator
@@ -20,8 +19,9 @@
 //   * every call looks up the array's device address in the current device's context
 //     (cudaGetSymbolAddress, a host-side query), so a context that was destroyed and
 //     created again (cudaDeviceReset) never leaves a stale address behind;
-//   * the call waits for its own work (it synchronises the stream and reads back the
-//     device error word), so it may not be called while any stream is capturing;
+//   * the call waits for its own work (it synchronises the stream, and reads back the device
+//     error word where its sort has a wait that can run out), so it may not be called while
+//     any stream is capturing;
 //   * a CUDA error left pending by earlier, unrelated work is not taken over: the call
 //     refuses to start and leaves that error in place for its owner.
 #include <cstdio>
