@@ -175,7 +175,8 @@ int tgpu_batch_program(const TgpuBatch *batch);
  *                  defaults of cell_multiple (1) and x_cell_factor (1/2), batches of more
  *                  than 16,384 agents whose program records pair lists (SPH) get cells of
  *                  1/2 to 1/4 of min_part_sizes where the agents are dense; any other pair
- *                  of values, and a rollout with gradients, uses the cells given
+ *                  of values uses the cells given (a rollout with gradients counts each
+ *                  instance's agents alone)
  *   union_factor   a warp walks the union of its seers' cell boxes (one read serves all
  *                  32 lanes) when that union is at most union_factor times the largest
  *                  single box; otherwise each lane walks its own box.  1 (the default; 0

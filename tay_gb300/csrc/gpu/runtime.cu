@@ -106,16 +106,6 @@ uint32_t next_pow2(uint32_t v) {
     return p;
 }
 
-// Agents per cell (with the default x cells of half the edge) that programs with a recording pass
-// aim at, and the agents of a batch from which they do (fill_multiple); fewer from kFineAgents on,
-// about where such programs go over to one lane per seer.  With the default rule's neighbours for
-// 64 agents per cubed part, us per step at a third / a quarter of the part size: 20,480 agents
-// 138 / 145, 40,960 229 / 236, 81,920 333 / 309, 131,072 415 / 372, 524,288 1299 / 1133.  Less dense
-// groups of 262,144 (1 / 2, 1 / 3, 1 / 4): 32 per cubed part 467, 446, 475; 21 316, 319, 347;
-// 15.6 288, 299, 325.
-constexpr float kFill = 32.0f / 27.0f, kFineFill = 0.72f;
-constexpr uint32_t kFillAgents = 16384, kFineAgents = 80000;
-
 // Largest segment that one launch boxes, keys and sorts, and largest that a cluster sorts with
 // a launch per radix pass (a change of the keys' width is then one launch more or less, as
 // with the general path); beyond, the general path spreads the work over more of the chip.
@@ -319,7 +309,7 @@ int tgpu::prepare_specs(TgpuBatch *b) {
     for (int s = 0; s < b->nseg; ++s) {
         SegmentSpec &sp = next[s];
         const HostSeg &h = b->hs[s];
-        sp.fill = b->fill;
+        sp.fill = sp.count > b->fill_least ? b->fill : 0.0f;
         uint32_t want[3] = {2, 2, 2};
         float exts[3];
         for (int a = 0; a < 3; ++a)

@@ -146,3 +146,30 @@ def test_replay_of_short_lists(gpu, most):
             api.set_tuning()
     assert got[0][:3] == got[1][:3]
     assert got[0][3] == (len(recs) + 127) // 128 * 4 and got[1][3] == 0  # every warp of every block
+
+
+def test_rollout_cells_depend_on_the_instance(gpu):
+    """Rollouts give instances above 16,384 particles cells below the part size, by their own
+    count: a large and a small instance have the same trajectories and gradients alone and
+    together, bit for bit."""
+    from tay_gb300.adjoint import SphRollout
+
+    def rollout(shapes):
+        inst = []
+        for shape in shapes:
+            s = W.sph_dam(*shape)
+            s.points.v[:, :3] = 0.02 * np.random.default_rng(shape[0]).standard_normal((s.points.n, 3))
+            inst.append((s.points, 0.05, 20.0, (0.0, 0.0, 0.0), (2.0, 1.5, 0.8)))
+        roll = SphRollout(inst, 4, checkpoint_every=2)
+        x, v = roll.forward()
+        dx, dv, dp = roll.backward(2.0 * x)
+        roll.close()
+        return x, dx, dv, dp
+
+    large, small = (32, 40, 16), (16, 16, 8)
+    both, a, b = rollout([large, small]), rollout([large]), rollout([small])
+    n = len(a[0])
+    for k in range(3):
+        assert both[k][:n].tobytes() == a[k].tobytes()
+        assert both[k][n:].tobytes() == b[k].tobytes()
+    assert both[3][0].tobytes() == a[3][0].tobytes() and both[3][1].tobytes() == b[3][0].tobytes()
