@@ -45,7 +45,10 @@ TGPU_D void fold_fn(Seer &s, const Term &t) {
 struct See {
     using Term = test_basic::Term;
     static constexpr bool kCheapTerm = true;
-    static constexpr int kLaneUnroll = 4;  // (100,000 agents: see pass 60 us at 2, 43 at 4, 46 at 8)
+    // Candidates in flight (see pass, us): 100,000 agents 60 at 2 (an earlier walk), 41.6 at 3, 37.8
+    // at 4, 36.2 at 5, 36.1 at 6; 200,000 at eight times the pairs 454, 367, 322, 314; 30,000 27.2 at
+    // 4, 24.3 at 6.  At 8 the left-over candidates of a row cost more (46 against 43 at 4, earlier).
+    static constexpr int kLaneUnroll = 6;
     static constexpr bool kSeenMinusSeer = true;  // d = b - a
     template <class Acc>
     TGPU_D static bool term(const Seer &, const float4 &a, const float4 &b, const Acc &, uint32_t, const SeeCtx &,
