@@ -1322,8 +1322,10 @@ __global__ void __launch_bounds__(kSeeThreads, see_detail::group_ctas<P>()) see_
 
     if (!replayed) {
         const bool recording = kList == 1 && !kBox && L.plist.mode == 1u;
-        const uint32_t ny = (uint32_t)(hi[1] - lo[1] + 1);
-        const uint32_t nrows = active ? ny * (uint32_t)(hi[2] - lo[2] + 1) : 0u;
+        // an inverted interval (a negative radius, a box whose max corner lies below its min
+        // corner) has no rows, as the loops of see_rows_kernel have none
+        const uint32_t ny = (uint32_t)max(hi[1] - lo[1] + 1, 0);
+        const uint32_t nrows = active ? ny * (uint32_t)max(hi[2] - lo[2] + 1, 0) : 0u;
         if (L.telemetry && lane == 0) atomicAdd(L.telemetry + 4, 1ull);
         uint32_t listed = 0;
         for (uint32_t rb = 0; __any_sync(0xffffffffu, rb < nrows); rb += kRows) {
@@ -1438,7 +1440,8 @@ __global__ void __launch_bounds__(kSeeThreads, see_detail::group_ctas<P>()) see_
                     uint32_t all = pairs;
 #pragma unroll
                     for (int o = 1; o < G; o <<= 1) all += __shfl_xor_sync(0xffffffffu, all, o);
-                    if (active && sub == 0) L.plist.count[i] = make_uint2(listed, all - own);
+                    // (a seer that walked no row did not meet itself)
+                    if (active && sub == 0) L.plist.count[i] = make_uint2(listed, all - min(all, own));
                 }
             }
             if (sub == 0 && L.skip_self) pairs -= own;

@@ -1,0 +1,132 @@
+"""GPU: values that no workload has but that the entry points take: negative and zero see
+radii, and box agents whose max corner lies below their min corner.  The reference's box test
+decides (a pair is skipped when |seer - seen| > r on an axis), so a negative radius on any axis
+of the space finds nothing, at every number of lanes per seer."""
+import ctypes
+import dataclasses
+
+import numpy as np
+import pytest
+
+from oracle import pyoracle as O
+from tay_gb300 import api
+from tay_gb300 import models as M
+from tay_gb300 import workloads as W
+
+pytestmark = pytest.mark.gpu
+
+# agents and neighbours per agent that give 32, 16, 8 and 1 lanes per seer
+SPACE = [(2500, 100), (5000, 100), (6000, 25), (20000, 100)]
+FLAT = [(2000, 100), (4000, 100), (2500, 10), (10000, 100)]
+
+
+def _side(n, mates, dims, radius=50.0):
+    return 2.0 * radius * (n / mates) ** (1.0 / dims)
+
+
+def _set_radii(b, radii):
+    for k in range(b._descs[0].pass_count):
+        b._descs[0].passes[k].radii[:] = list(radii) + [0.0]
+    b._check(b.L.tgpu_batch_set_contexts(b.ptr, 0, ctypes.byref(b._descs[0])), "tgpu_batch_set_contexts")
+
+
+@pytest.mark.parametrize("dims,n,mates", [(3, *x) for x in SPACE] + [(2, *x) for x in FLAT] + [(1, *x) for x in FLAT])
+def test_negative_radii_find_nothing(gpu, dims, n, mates):
+    """Radii set to negative ones between runs (the batch keeps the lanes of its first run)."""
+    ps = W.basic_points(n, seed=71, side=_side(n, mates, dims))
+    recs = M.records(M.TEST_RECORD, ps.p, ps.v)
+    setup = dataclasses.replace(M.test_setup(passes=("agent_see",), mb=16), dims=dims)
+    b = api.Batch([(setup, recs)])
+    try:
+        b.push()
+        pairs = b.run(1)[1]
+        assert pairs > 0
+        first = b.fetch(0).tobytes()
+        for axis in range(dims):
+            for r in (-1e-3, -1.0, -60.0, -1e6, -np.inf):
+                radii = [50.0, 50.0, 50.0]
+                radii[axis] = r
+                _set_radii(b, radii)
+                assert b.run(1)[1] == 0, radii
+        for radii in ([-50.0] * 3, [-1.0, -60.0, -1e6]):
+            _set_radii(b, radii)
+            assert b.run(1)[1] == 0, radii
+        assert M.by_id(b.fetch(0)).tobytes() == M.by_id(np.frombuffer(first, M.TEST_RECORD)).tobytes()
+        _set_radii(b, [50.0] * 3)
+        assert b.run(1)[1] == pairs
+    finally:
+        b.close()
+
+
+@pytest.mark.parametrize("dims,n,mates", [(3, *SPACE[0])] + [(2, *x) for x in FLAT])
+def test_states_of_negative_radius(gpu, dims, n, mates):
+    ps = W.basic_points(n, seed=72, side=_side(n, mates, dims))
+    recs = M.records(M.TEST_RECORD, ps.p, ps.v)
+    setup = dataclasses.replace(M.test_setup(radius=-50.0, passes=("agent_see",), mb=16), dims=dims)
+    b = api.Batch([(setup, recs)])
+    try:
+        b.push()
+        assert b.run(1)[1] == 0
+        assert not b.fetch(0)["b_buffer_count"].any()
+    finally:
+        b.close()
+
+
+@pytest.mark.parametrize("n", [2000, 5000, 20000, 40000])
+def test_recorded_lists_of_negative_radius(gpu, n):
+    """SPH: the density pass records empty lists and the force pass replays them."""
+    side = int(np.ceil(n ** (1 / 3)))
+    sph = W.sph_dam(side, side, side)
+    setup = M.sph_setup(passes=("sph_density", "sph_pressure", "sph_force"), mb=64)
+    recs = M.records(M.SPH_RECORD, sph.points.p[:n], sph.points.v[:n])
+    b = api.Batch([(setup, recs)])
+    try:
+        b.push()
+        assert b.run(1)[1] > 0
+        for axis in range(3):
+            radii = [0.04, 0.04, 0.04]
+            radii[axis] = -0.3
+            _set_radii(b, radii)
+            assert b.run(1)[1] == 0
+            got = b.fetch(0)
+            assert not got["rho"].any() and not got["a"].any()
+    finally:
+        b.close()
+
+
+@pytest.mark.parametrize("n,mates", SPACE[:3] + [(31000, 100)])
+def test_inverted_boxes(gpu, port, n, mates):
+    """A box whose max corner lies far below its min corner, on one axis or on all: exact counts."""
+    w = W.box_agents(n, seed=73, side=_side(n, mates, 3))
+    for k in range(7):
+        axes = [k] if k < 3 else [0, 1, 2]
+        for a in axes:
+            w.hi[k::28, a] = w.lo[k::28, a] - 400.0 * (k + 1)
+    recs = M.box_records(w.lo, w.hi, w.v)
+    setup = M.box_setup(passes=("box_agent_see",), mb=16)
+    b = api.Batch([(setup, recs)])
+    try:
+        b.push()
+        b.run(1)
+        got = M.by_id(b.fetch(0))
+    finally:
+        b.close()
+    want = port.run(O.MODEL_BOX, "simple", recs, setup.passes[0].ctx, setup.passes[0].ctx, 50.0, 50.0, 1,
+                    O.PASS_SEE0).records
+    assert got["b_buffer_count"].sum() > 0
+    assert np.array_equal(got["b_buffer_count"], want["b_buffer_count"])
+
+
+@pytest.mark.parametrize("n", [1, 1000, 5000, 20000, 65536])
+def test_allocation_free_pass_of_negative_radius(gpu, n):
+    torch = pytest.importorskip("torch")
+    L = api.lib()
+    pos = torch.from_numpy(W.basic_points(n, seed=74).p.copy()).cuda()
+    parts = (ctypes.c_float * 4)(50.0, 50.0, 50.0, 50.0)
+    for radii in ((50.0, 50.0, -1.0), (50.0, -300.0, 50.0), (-1e6, 50.0, 50.0), (-50.0, -50.0, -50.0)):
+        out = torch.full((n, 4), -1.0, dtype=torch.float32, device="cuda")
+        torch.cuda.synchronize()
+        rc = L.tgpu_see_noalloc(ctypes.c_void_p(pos.data_ptr()), n, (ctypes.c_float * 4)(*radii, 0.0), parts,
+                                ctypes.c_void_p(out.data_ptr()), None)
+        assert rc == 0, L.tgpu_noalloc_last_error().decode()
+        assert not out.cpu().numpy().any(), radii
