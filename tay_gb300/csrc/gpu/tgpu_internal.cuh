@@ -258,12 +258,12 @@ TGPU_HD uint32_t cell_key(const SegmentSpec &s, uint32_t x, uint32_t y, uint32_t
 // A segment's grid for one step with its rounding pad, derived once per step from the
 // bounding box (derive_grid) and read by every later kernel of the step.  The pad is a bound
 // of the rounding error, in cells, of a cell coordinate computed as
-// floor((p - origin) * inv_cs) and of a search interval's ends: 16 ulps of the largest
-// coordinate magnitude (p - r, less the origin, and p - origin round by half an ulp each), plus
-// 4 * 2^-23 of the largest cell coordinate (the rounding of inv_cs and of the product: 1.5 *
-// 2^-23).  No wider than that: with cells of the see radius a seer whose interval crosses one
-// more cell border makes its whole warp walk another row of cells on each side, and a pad of
-// 1/512 cell put one in 256 seers there (see pass of 100,000 test agents 42.7 against 34.5 us).
+// floor((p - origin) * inv_cs): 16 ulps of the largest coordinate magnitude (p - origin rounds
+// by half an ulp), plus 4 * 2^-23 of the largest cell coordinate (the rounding of inv_cs and of
+// the product: 1.5 * 2^-23).  What a seer's own magnitudes add, axis_span (see.cuh) adds.  No
+// wider than that: with cells of the see radius a seer whose interval crosses one more cell
+// border makes its whole warp walk another row of cells on each side, and a pad of 1/512 cell
+// put one in 256 seers there (see pass of 100,000 test agents 42.7 against 37.8 us).
 struct SegGrid {
     Grid g;
     float pad;

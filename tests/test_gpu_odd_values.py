@@ -130,3 +130,67 @@ def test_allocation_free_pass_of_negative_radius(gpu, n):
                                 ctypes.c_void_p(out.data_ptr()), None)
         assert rc == 0, L.tgpu_noalloc_last_error().decode()
         assert not out.cpu().numpy().any(), radii
+
+
+def _far_seers(rng, n, radius, edge=0.0):
+    """Seers whose search interval [p - radius, p + radius] ends inside [0, 5], half of them from
+    each side; the other axes near 0."""
+    u = rng.uniform(0.0, 5.0, n)
+    p = np.zeros((n, 4), np.float32)
+    p[:, 0] = np.where(np.arange(n) % 2, radius + edge + u, u - radius)
+    p[:, 1:3] = rng.uniform(0.0, 0.004, (n, 2))
+    return p
+
+
+@pytest.mark.parametrize("radius", [1e4, 1e5])
+@pytest.mark.parametrize("tuning", [{}, {"hit_masks": 1}, {"cell_order": 0, "cell_multiple": 0.5}])
+def test_far_seers_of_another_group(gpu, radius, tuning):
+    """Seers one radius away from a small group with fine cells: their coordinates, and the
+    differences of the box test, round more coarsely than the group's cells.  Exact counts
+    against the box test in float32 over all pairs."""
+    rng = np.random.default_rng(75)
+    seen = np.zeros((3000, 4), np.float32)
+    seen[:, :3] = rng.uniform(0.0, 1.0, (3000, 3)) * [5.0, 0.004, 0.004]
+    seers = _far_seers(rng, 4000, radius)
+    r = np.float32(radius)
+    want = np.ones((4000, 3000), bool)
+    for a in range(3):
+        want &= np.abs(seers[:, None, a] - seen[None, :, a]) <= r
+    see, act = M.test_contexts(radius)
+    zero = [np.zeros_like(x) for x in (seers, seen)]
+    recs = [M.records(M.TEST_RECORD, x, v) for x, v in zip((seers, seen), zero)]
+    api.set_tuning(**tuning)
+    try:
+        got = M.run_groups(M.TEST_RECORD, ("agent_see", "agent_act"), recs, [("see", 0, 1, False)], see, act, radius,
+                           0.01, 1)
+    finally:
+        api.set_tuning()
+    assert np.array_equal(got[0]["b_buffer_count"], want.sum(1))
+
+
+@pytest.mark.parametrize("radius", [1e4, 1e5])
+@pytest.mark.parametrize("tuning", [{}, {"cell_order": 0, "cell_multiple": 0.5}])
+def test_far_boxes_of_another_group(gpu, radius, tuning):
+    rng = np.random.default_rng(76)
+
+    def box(lo, edge):
+        hi = lo.copy()
+        hi[:, :3] += np.float32(edge)
+        return lo, hi
+
+    lo = np.zeros((3000, 4), np.float32)
+    lo[:, :3] = rng.uniform(0.0, 1.0, (3000, 3)) * [5.0, 0.004, 0.004]
+    seen, seers = box(lo, 0.5), box(_far_seers(rng, 4000, radius, 0.5), 0.0)
+    r = np.float32(radius)
+    want = np.ones((4000, 3000), bool)
+    for a in range(3):
+        want &= ~(seers[0][:, None, a] - seen[1][None, :, a] > r) & ~(seen[0][None, :, a] - seers[1][:, None, a] > r)
+    see, act = M.test_contexts(radius)
+    recs = [M.box_records(x, y, np.zeros_like(x)) for x, y in (seers, seen)]
+    api.set_tuning(**tuning)
+    try:
+        got = M.run_groups(M.BOX_RECORD, ("box_agent_see", "box_agent_act"), recs, [("see", 0, 1, False)], see, act,
+                           radius, 0.01, 1, is_point=False)
+    finally:
+        api.set_tuning()
+    assert np.array_equal(got[0]["b_buffer_count"], want.sum(1))
