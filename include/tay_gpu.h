@@ -172,11 +172,13 @@ int tgpu_batch_program(const TgpuBatch *batch);
  *   stage_cap      agents staged per CTA (0 = default)
  *   stage_cells    halo cells per CTA (0 = default)
  *   cell_multiple  grid cell edge = cell_multiple x min_part_sizes (0 = 1).  With the
- *                  defaults of cell_multiple (1) and x_cell_factor (1/2), batches of more
+ *                  defaults of cell_multiple (1) and x_cell_factor (1/2), groups of more
  *                  than 16,384 agents whose program records pair lists (SPH) get cells of
- *                  1/2 to 1/4 of min_part_sizes where the agents are dense; any other pair
- *                  of values uses the cells given (a rollout with gradients counts each
- *                  instance's agents alone)
+ *                  1/2 to 1/4 of min_part_sizes where the agents are dense, by the group's
+ *                  own agents: a state steps alone, in a batch and in a rollout with
+ *                  gradients through the same bits (a batch whose tables of such cells
+ *                  cannot be allocated keeps min_part_sizes for all its groups).  Any other
+ *                  pair of values uses the cells given
  *   union_factor   a warp walks the union of its seers' cell boxes (one read serves all
  *                  32 lanes) when that union is at most union_factor times the largest
  *                  single box; otherwise each lane walks its own box.  1 (the default; 0

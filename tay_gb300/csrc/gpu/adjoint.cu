@@ -338,16 +338,6 @@ int tgpu_adjoint_create(TgpuBatch *b, int steps, int checkpoint_every, int keep_
     if (b->m != model_sph() || b->program != 3)
         return fail(TGPU_ERR_PROGRAM, "adjoint: the batch must run the full SPH sequence "
                                       "(sph_density, sph_pressure, sph_force, sph_integrate)");
-    // A rollout's cells depend on each instance alone: other cells sum in another order, and its
-    // gradients, which add up the rounding of every step, would change with the number of
-    // particles it is batched with.  Instances below kFillAgents keep the part size, larger ones
-    // get the cells of large batches (32 x 20,480 particles over 200 steps: recorded forward
-    // 483 -> 366 ms, backward 728 -> 608).
-    if (b->fill > 0.0f) {
-        b->specs_dirty = true;
-        b->fill = kFineFill;
-        b->fill_least = kFillAgents;
-    }
     int rc = prepare_specs(b);
     if (rc) return rc;
     TgpuAdjoint *a = new TgpuAdjoint();

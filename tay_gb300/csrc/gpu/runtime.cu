@@ -309,7 +309,7 @@ int tgpu::prepare_specs(TgpuBatch *b) {
     for (int s = 0; s < b->nseg; ++s) {
         SegmentSpec &sp = next[s];
         const HostSeg &h = b->hs[s];
-        sp.fill = sp.count > b->fill_least ? b->fill : 0.0f;
+        sp.fill = b->small_cells ? segment_fill(sp.count) : 0.0f;
         uint32_t want[3] = {2, 2, 2};
         float exts[3];
         for (int a = 0; a < 3; ++a)
@@ -347,11 +347,11 @@ int tgpu::prepare_specs(TgpuBatch *b) {
     }
     // tables of smaller cells that cannot be had: the part size's
     auto coarser = [b]() {
-        b->fill = 0.0f;
+        b->small_cells = false;
         b->specs_dirty = true;
         return prepare_specs(b);
     };
-    if (table_total > 0xFFFFFFFFull && b->fill > 0.0f) return coarser();
+    if (table_total > 0xFFFFFFFFull && b->small_cells) return coarser();
     if (table_total > 0xFFFFFFFFull)
         return fail(TGPU_ERR_ARG, "cell tables too large (%llu entries)", (unsigned long long)table_total);
     const uint32_t key_bits = max_key_bits;
@@ -363,7 +363,7 @@ int tgpu::prepare_specs(TgpuBatch *b) {
         b->table = nullptr;
         b->table_entries = 0;
         const cudaError_t e = cudaMalloc(&b->table, table_total * sizeof(uint2));
-        if (e == cudaErrorMemoryAllocation && b->fill > 0.0f) {
+        if (e == cudaErrorMemoryAllocation && b->small_cells) {
             cudaGetLastError();
             b->table = nullptr;
             return coarser();
@@ -1136,8 +1136,7 @@ int tgpu_batch_create(const TgpuGroup *groups, int group_count, TgpuBatch **out)
         g_tuning.cell_multiple != standard.cell_multiple || g_tuning.x_cell_factor != standard.x_cell_factor;
     bool records = false;
     for (int k = 0; k < pd.kernels; ++k) records = records || m->kernels[pd.kernel_index[k]].pair_list == 1;
-    if (records && !own_cells && b->cell_order == kOrderRows && b->total > kFillAgents)
-        b->fill = b->total > kFineAgents ? kFineFill : kFill;
+    b->small_cells = records && !own_cells && b->cell_order == kOrderRows;
     int cursor = 0;
     for (int k = 0; k < pd.kernels && !rc; ++k) {
         KernelRun r{};

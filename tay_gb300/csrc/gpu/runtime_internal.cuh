@@ -18,15 +18,21 @@ constexpr int kStatusWords = 10;
 // Segments up to which a row-order step clears its table with one memset per segment.
 constexpr int kMemsetClearSegments = 4;
 
-// Agents per cell (with the default x cells of half the edge) that programs with a recording pass
-// aim at, and the agents of a batch from which they do (fill_multiple); fewer from kFineAgents on,
-// about where such programs go over to one lane per seer.  With the default rule's neighbours for
-// 64 agents per cubed part, us per step at a third / a quarter of the part size: 20,480 agents
-// 138 / 145, 40,960 229 / 236, 81,920 333 / 309, 131,072 415 / 372, 524,288 1299 / 1133.  Less dense
-// groups of 262,144 (1 / 2, 1 / 3, 1 / 4): 32 per cubed part 467, 446, 475; 21 316, 319, 347;
-// 15.6 288, 299, 325.
+// Agents per cell (with the default x cells of half the edge) that a segment of `count` agents
+// aims at in programs with a recording pass (fill_multiple); 0: cells of the part size.  By the
+// segment's own count and nothing else: other cells sum in another order, and the bits of a
+// state must not depend on what it is batched with, nor on whether its batch records a rollout.
+// With the default rule's neighbours for 64 agents per cubed part, us per step at a third / a
+// quarter of the part size: 20,480 agents 138 / 145, 40,960 229 / 236, 81,920 333 / 309, 131,072
+// 415 / 372, 524,288 1299 / 1133.  Less dense groups of 262,144 (1 / 2, 1 / 3, 1 / 4): 32 per
+// cubed part 467, 446, 475; 21 316, 319, 347; 15.6 288, 299, 325.  Batches of small states do not
+// decide it: steps of 4 and 32 x 20,480 agents 364 / 391 and 1707 / 1760 us, 40 recorded and 40
+// backward steps of 32 x 20,480 62.3 / 57.9 and 84.6 / 79.8 ms.
 constexpr float kFill = 32.0f / 27.0f, kFineFill = 0.72f;
 constexpr uint32_t kFillAgents = 16384, kFineAgents = 80000;
+inline float segment_fill(uint32_t count) {
+    return count > kFineAgents ? kFineFill : count > kFillAgents ? kFill : 0.0f;
+}
 
 // Device buffers of one object in one allocation: add() every buffer, then one allocate(); each
 // starts on a 256-byte boundary.  (An object of a hundred buffers spent milliseconds in
@@ -110,8 +116,7 @@ struct TgpuBatch {
     uint32_t tiles = 0, ctas = 0, key_bits = 0;
     uint32_t cluster_blocks = 0, cluster_items = 0, cluster_split = 0;  // SortLaunch's
     bool specs_dirty = true;
-    float fill = 0.0f;        // SegmentSpec::fill of every segment
-    uint32_t fill_least = 0;  // of more agents than this
+    bool small_cells = false;  // segments may have cells below the part size (segment_fill)
 
     SegmentSpec *d_specs = nullptr;
     uint32_t *d_tile_seg = nullptr;
