@@ -426,6 +426,7 @@ int tgpu_adjoint_backward(TgpuAdjoint *a, const float *dl_dpos, const float *dl_
                           double *dparams) {
     if (!a || !a->recorded) return fail(TGPU_ERR_ARG, "adjoint: run tgpu_adjoint_forward first");
     TgpuBatch *b = a->b;
+    if (!b->table) return fail(TGPU_ERR_CUDA, "adjoint: the batch lost its cell table (a larger one failed to allocate)");
     const size_t n = b->total;
     cudaStream_t st = b->st;
     cudaMemsetAsync(a->xbar_id, 0, n * sizeof(float4), st);

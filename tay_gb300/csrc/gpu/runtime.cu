@@ -298,10 +298,11 @@ uint32_t tgpu::seer_lanes(uint64_t seers, double mates, int dims, bool boxes, bo
 
 // Per-segment grid bounds from the pushed agents: each axis gets a power-of-two cell
 // budget with 10% headroom over the pushed extent (bounded to 1024, the 10-bit Morton
-// limit); the dense table gets at most shared_megabytes of uint2 entries.
+// limit); the dense table gets at most shared_megabytes of uint2 entries.  After an error the
+// batch has not been prepared: no captured step of it is left that reads a table it no longer
+// has, and the next call tries again.
 int tgpu::prepare_specs(TgpuBatch *b) {
     if (!b->specs_dirty) return TGPU_OK;
-    b->specs_dirty = false;
     set_lanes(b);
     std::vector<SegmentSpec> next = b->specs;
     uint64_t table_total = 0;
@@ -348,7 +349,6 @@ int tgpu::prepare_specs(TgpuBatch *b) {
     // tables of smaller cells that cannot be had: the part size's
     auto coarser = [b]() {
         b->small_cells = false;
-        b->specs_dirty = true;
         return prepare_specs(b);
     };
     if (table_total > 0xFFFFFFFFull && b->small_cells) return coarser();
@@ -357,26 +357,31 @@ int tgpu::prepare_specs(TgpuBatch *b) {
     const uint32_t key_bits = max_key_bits;
     const bool same = b->table && key_bits == b->key_bits &&
                       !memcmp(next.data(), b->specs.data(), sizeof(SegmentSpec) * b->nseg);
-    if (same) return TGPU_OK;  // the table is left clean by every completed step
+    if (same) {  // the table is left clean by every completed step
+        b->specs_dirty = false;
+        return TGPU_OK;
+    }
+    for (auto &kv : b->graphs) cudaGraphExecDestroy(kv.second);
+    b->graphs.clear();
     if (table_total > b->table_entries) {
         cudaFree(b->table);
         b->table = nullptr;
         b->table_entries = 0;
         const cudaError_t e = cudaMalloc(&b->table, table_total * sizeof(uint2));
-        if (e == cudaErrorMemoryAllocation && b->small_cells) {
+        if (e != cudaSuccess) {
             cudaGetLastError();
             b->table = nullptr;
-            return coarser();
+            if (e == cudaErrorMemoryAllocation && b->small_cells) return coarser();
+            return fail(TGPU_ERR_CUDA, "cell tables of %llu entries: cudaMalloc failed: %s",
+                        (unsigned long long)table_total, cudaGetErrorString(e));
         }
-        CK(e);
         b->table_entries = table_total;
     }
+    CK(cudaMemsetAsync(b->table, 0, b->table_entries * sizeof(uint2), b->st));
+    CK(cudaMemcpyAsync(b->d_specs, next.data(), sizeof(SegmentSpec) * b->nseg, cudaMemcpyHostToDevice, b->st));
     b->specs = next;
     b->key_bits = key_bits;
-    CK(cudaMemsetAsync(b->table, 0, b->table_entries * sizeof(uint2), b->st));
-    CK(cudaMemcpyAsync(b->d_specs, b->specs.data(), sizeof(SegmentSpec) * b->nseg, cudaMemcpyHostToDevice, b->st));
-    for (auto &kv : b->graphs) cudaGraphExecDestroy(kv.second);
-    b->graphs.clear();
+    b->specs_dirty = false;
     // box reset, bounding box (+ grids), keys and histograms (+ digit offsets), one kernel
     // per radix pass (or one kernel for all of these, or per pass), cell table (+ reorder), the passes, and the table clear when it is
     // a kernel (Morton order, or more segments than separate header memsets)
