@@ -933,22 +933,30 @@ bool cluster_sort_shape(uint32_t segments, uint32_t largest, uint32_t most_agent
     *blocks = 0;
     *items = 0;
     if (!segments || largest > most_agents) return false;
-    // 2 agents a thread (2,048 a block) as long as the blocks last, then 4, then 8
+    // 2 agents a thread (2,048 a block), else 4, else 8: the first whose clusters, one a segment,
+    // the device holds at once (152 blocks in clusters of 1 or 2, but 144, 120 and 112 in clusters
+    // of 4, 8 and 16).  A second wave costs a whole sort, more agents a thread less: 16 segments
+    // of 16,384 agents take 44 us at 2 a thread in two waves, 32 at 4 in one, 63 by the general
+    // path; 8 of 131,072 91 us in two waves at 8 a thread, 94 by the general path, whose passes
+    // leave the step shorter (253 against 261 us).
     SortLaunch L{};
     L.segments = segments;
-    L.cluster_items = 2;
-    while (L.cluster_items < 8u && largest > kClusterMost * L.cluster_items * kClusterThreads) L.cluster_items *= 2;
-    L.cluster_blocks = 1;
-    while (L.cluster_blocks * L.cluster_items * kClusterThreads < largest) L.cluster_blocks *= 2;
-    if (L.cluster_blocks > kClusterMost || segments * L.cluster_blocks > kClusterWave) return false;
-    int clusters = 0;
-    if (cluster_sort(L, false, nullptr, &clusters) != cudaSuccess || clusters < 1) {
-        cudaGetLastError();
-        return false;
+    for (L.cluster_items = 2; L.cluster_items <= 8u; L.cluster_items *= 2) {
+        L.cluster_blocks = 1;
+        while (L.cluster_blocks * L.cluster_items * kClusterThreads < largest) L.cluster_blocks *= 2;
+        if (L.cluster_blocks > kClusterMost) continue;
+        int clusters = 0;
+        if (cluster_sort(L, false, nullptr, &clusters) != cudaSuccess) {
+            cudaGetLastError();
+            return false;
+        }
+        if (clusters > 0 && (uint32_t)clusters >= segments) {
+            *blocks = L.cluster_blocks;
+            *items = L.cluster_items;
+            return true;
+        }
     }
-    *blocks = L.cluster_blocks;
-    *items = L.cluster_items;
-    return true;
+    return false;
 }
 
 void launch_cluster_sort(const SortLaunch &L, cudaStream_t st, uint32_t **sorted_keys, uint32_t **perm) {

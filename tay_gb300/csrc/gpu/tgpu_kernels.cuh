@@ -146,9 +146,8 @@ constexpr size_t sort_scratch_bytes(uint32_t segments, uint32_t tiles) {
 void launch_sort(const SortLaunch &L, cudaStream_t st, uint32_t **sorted_keys, uint32_t **perm);
 // Boxes, grids, keys and sort of small segments in one launch (cluster_sort_kernel), in place
 // of launch_box and launch_sort.  cluster_sort_shape: whether it takes `segments` segments of
-// at most `largest` agents (not more than most_agents, nor more blocks than one wave), and
-// with how many blocks per segment and agents per thread; also prepares its launch.
-constexpr uint32_t kClusterWave = 152;
+// at most `largest` agents (not more than most_agents, nor more clusters than the device runs
+// at once), and with how many blocks per segment and agents per thread; also prepares its launch.
 bool cluster_sort_shape(uint32_t segments, uint32_t largest, uint32_t most_agents, uint32_t *blocks, uint32_t *items);
 void launch_cluster_sort(const SortLaunch &L, cudaStream_t st, uint32_t **sorted_keys, uint32_t **perm);
 // Writes (write_runs = 1) or clears (0) the cell table of the sorted keys.  With `set`, the
