@@ -71,7 +71,10 @@ struct BoxAcc {
 
 TGPU_HD uint32_t float_to_ordered(float f) {
 #ifdef __CUDA_ARCH__
-    uint32_t b = __float_as_uint(f);
+    // (moved by PTX: seen as a float, setting the sign bit may be compiled as -|f|, which gives
+    // a NaN back without its sign and so the encoding of -0)
+    uint32_t b;
+    asm("mov.b32 %0, %1;" : "=r"(b) : "f"(f));
 #else
     union { float f; uint32_t u; } cvt;
     cvt.f = f;

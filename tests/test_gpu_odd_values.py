@@ -194,3 +194,92 @@ def test_far_boxes_of_another_group(gpu, radius, tuning):
     finally:
         api.set_tuning()
     assert np.array_equal(got[0]["b_buffer_count"], want.sum(1))
+
+
+def _odd_records(model, n, kind, fixed):
+    """A workload with positions (boxes: corners) that are NaN or infinite, on one axis or all."""
+    if model == "box":
+        w = W.box_agents(n, seed=81, side=_side(n, 100, 3))
+        setup, corners, side = M.box_setup(mb=16), (w.lo, w.hi), _side(n, 100, 3)
+    elif model == "sph":
+        e = int(np.ceil(n ** (1 / 3)))
+        w = W.sph_dam(e, e, e).points
+        setup, corners, side = M.sph_setup(mb=16), (w.p[:n],), 0.01 * e
+    elif model == "boids":
+        side = (125.0 * n) ** (1 / 3)
+        w = W.basic_points(n, seed=82, side=side)
+        setup, corners = M.boids_setup(mb=16), (w.p,)
+    else:
+        side = _side(n, 100, 3)
+        w = W.basic_points(n, seed=83, side=side)
+        setup, corners = M.test_setup(mb=16), (w.p,)
+    values = [np.nan] if kind == "nan" else [np.inf, -np.inf, np.nan]
+    for k, axes in enumerate(([0], [1], [2], [0, 1, 2], [0, 2])):
+        for c in corners:
+            c[k::977, axes] = values[k % len(values)]
+    if len(corners) == 2:
+        corners[1][5::977, 1] = np.inf  # a box without an upper end
+    if fixed:
+        setup = dataclasses.replace(setup, fixed_box=((0.0, 0.0, 0.0), (side, side, side)))
+    if model == "box":
+        return setup, M.box_records(*corners, w.v)
+    return setup, M.records(setup.dtype, corners[0], w.v[:n])
+
+
+def _same(a, b):
+    """Equal values in every field, NaNs of any payload equal."""
+    for f in a.dtype.names:
+        x, y = a[f], b[f]
+        if x.dtype.kind == "f" or (x.dtype.subdtype and x.dtype.subdtype[0].kind == "f"):
+            assert np.array_equal(x, y, equal_nan=True), f
+        else:
+            assert np.array_equal(x, y), f
+
+
+def _run_odd(groups, steps):
+    b = api.Batch(groups)
+    try:
+        b.push()
+        pairs = b.run(steps)[1]
+        return M.by_id(b.fetch(0)), pairs, b.launches_per_step()
+    finally:
+        b.close()
+
+
+@pytest.mark.parametrize("fixed", [False, True])
+@pytest.mark.parametrize("kind", ["nan", "inf"])
+@pytest.mark.parametrize("model,n", [("test", 2500), ("test", 5001), ("test", 20000), ("box", 3001), ("box", 12289),
+                                     ("boids", 2049), ("boids", 8193), ("sph", 4097), ("sph", 20001)])
+def test_nan_and_infinite_positions(gpu, model, n, kind, fixed):
+    """A state alone (shared lanes, cluster sort) and in a batch of so many agents and segments
+    that every seer has one lane and the sort is the general one; the agents beside it are
+    scattered over a large space.  The second step meets the NaNs that the first one computed."""
+    setup, recs = _odd_records(model, n, kind, fixed)
+    plain = dataclasses.replace(setup, fixed_box=None)
+    x = W.basic_points(60000, seed=85, side=5000.0)
+    if model == "box":
+        other = M.box_records(x.p, x.p, x.v)
+    else:
+        other = M.records(setup.dtype, x.p, x.v)
+    many = [(plain, other)] + [(plain, other[:5])] * 200
+    for steps in (1, 2):
+        got, pairs, launches = _run_odd([(setup, recs)], steps)
+        want, _, general = _run_odd([(setup, recs)] + many, steps)
+        assert pairs > 0 and launches < general
+        _same(got, want)
+
+
+@pytest.mark.parametrize("n,mates", SPACE)
+def test_zero_radius(gpu, n, mates):
+    """Neighbours are the agents in exactly the same place."""
+    ps = W.basic_points(n, seed=84, side=_side(n, mates, 3))
+    ps.p[n // 2:2 * (n // 2)] = ps.p[:n // 2]
+    recs = M.records(M.TEST_RECORD, ps.p, ps.v)
+    b = api.Batch([(M.test_setup(passes=("agent_see",), mb=16), recs)])
+    try:
+        b.push()
+        assert b.run(1)[1] > 0
+        _set_radii(b, [0.0] * 3)
+        assert b.run(1)[1] == 2 * (n // 2)
+    finally:
+        b.close()
