@@ -47,28 +47,29 @@ TGPU_D uint32_t warp_sum_u(uint32_t v) {
     return v;
 }
 
+// A radius (or an edge) with what the differences that are tested against it may round away: half
+// an ulp of it.
+TGPU_D float rounded_out(float r) { return r * 1.00000024f; }  // 1 + 2^-22
+
 // Cell range along one axis for the interval [lo_v, hi_v] (a seer's search interval over the
-// seen agents' positions), widened on each side so that rounding can never put a neighbour that
-// passes the box test outside the range: by `pad` cells (SegGrid: the rounding of the seen
-// agents' cell coordinates) and by four half-ulps, 2^-22, of `size`, the sum of the magnitudes
-// that the interval's ends and the box test's differences are rounded at (the seer's coordinate,
-// the radius, for boxes the largest edge: 2 + 3 + 2 halves of an ulp at most).  A seer of
-// another group can lie far outside the grid that it searches, where `pad` says nothing: seers
-// 10,000 away from a group 5 across with cells of 1/200 lost 51 of 6 million pairs.
-// (An infinite size widens by a finite width, so an infinite end stays where it is.)
-TGPU_D void axis_span(float lo_v, float hi_v, float size, float origin, float inv_cs, int dim, float pad, int &lo,
-                      int &hi) {
-    const float w = pad + fminf(size * inv_cs * 2.384185791e-7f, 3.0e38f);
-    float a = (lo_v - origin) * inv_cs - w;
-    float b = (hi_v - origin) * inv_cs + w;
+// seen agents' positions, its ends rounded outwards), widened by `pad` cells on each side
+// (SegGrid: the rounding of cell coordinates), so that rounding can never put a neighbour that
+// passes the box test outside the range.
+TGPU_D void axis_span(float lo_v, float hi_v, float origin, float inv_cs, int dim, float pad, int &lo, int &hi) {
+    float a = (lo_v - origin) * inv_cs - pad;
+    float b = (hi_v - origin) * inv_cs + pad;
     int l = (int)floorf(a), h = (int)floorf(b);
     lo = l < 0 ? 0 : (l >= dim ? dim - 1 : l);
     hi = h < 0 ? 0 : (h >= dim ? dim - 1 : h);
 }
 
-// The same for the interval [p - r, p + r].
+// The same for the interval [p - r, p + r].  Rounded to nearest, its ends and the differences
+// of the box test are off by ulps of p and r, and for a seer of another group, which can lie far
+// outside the grid that it searches, `pad` says nothing about those: seers 10,000 away from a
+// group 5 across with cells of 1/200 lost 51 of 6 million pairs.
 TGPU_D void axis_range(float p, float r, float origin, float inv_cs, int dim, float pad, int &lo, int &hi) {
-    axis_span(p - r, p + r, fabsf(p) + fabsf(r), origin, inv_cs, dim, pad, lo, hi);
+    r = rounded_out(r);
+    axis_span(__fsub_rd(p, r), __fadd_ru(p, r), origin, inv_cs, dim, pad, lo, hi);
 }
 
 // Non-point seer over non-point seen agents (tay/space.c:92-103): skipped when on any
@@ -516,8 +517,9 @@ TGPU_D void seer_cells(const float4 &sp, const float4 &smax, const float4 &r4, c
     }
     const float sx = ordered_to_float(B.size[0]), sy = ordered_to_float(B.size[1]), sz = ordered_to_float(B.size[2]);
     auto axis = [&](float mn, float mx, float r, float edge, int a) {
-        axis_span((mn - r) - edge, mx + r, fmaxf(fabsf(mn), fabsf(mx)) + fabsf(r) + edge, g.origin[a], g.inv_cs[a],
-                  g.dims[a], pad, lo[a], hi[a]);
+        r = rounded_out(r);
+        axis_span(__fsub_rd(__fsub_rd(mn, r), rounded_out(edge)), __fadd_ru(mx, r), g.origin[a], g.inv_cs[a], g.dims[a],
+                  pad, lo[a], hi[a]);
     };
     axis(sp.x, smax.x, r4.x, sx, 0);
     axis(sp.y, smax.y, r4.y, sy, 1);

@@ -263,7 +263,7 @@ TGPU_HD uint32_t cell_key(const SegmentSpec &s, uint32_t x, uint32_t y, uint32_t
 // of the rounding error, in cells, of a cell coordinate computed as
 // floor((p - origin) * inv_cs): 16 ulps of the largest coordinate magnitude (p - origin rounds
 // by half an ulp), plus 4 * 2^-23 of the largest cell coordinate (the rounding of inv_cs and of
-// the product: 1.5 * 2^-23).  What a seer's own magnitudes add, axis_span (see.cuh) adds.  No
+// the product: 1.5 * 2^-23); a seer's interval is rounded outwards (axis_range, see.cuh).  No
 // wider than that: with cells of the see radius a seer whose interval crosses one more cell
 // border makes its whole warp walk another row of cells on each side, and a pad of 1/512 cell
 // put one in 256 seers there (see pass of 100,000 test agents 42.7 against 37.8 us).
