@@ -259,6 +259,10 @@ unsigned long long tgpu_batch_device_bytes(const TgpuBatch *batch);
  * min_part_sizes are 4 host floats each.  All intermediate buffers live in one fixed
  * array (about 4 MB) of the library's own device memory, which every GPU that loads the
  * library holds until the process exits; no device memory is allocated.
+ *   - the call sees no density before it runs, so its launch shape (lanes per agent) goes by n
+ *     alone, for some 100 neighbours per agent; results do not depend on it, but well above
+ *     15,000 agents with several hundred neighbours each, or with next to none below, a
+ *     batch's pass over the same positions picks a better one;
  *   - n must not exceed tgpu_noalloc_max_agents() (65536); larger calls fail with
  *     TGPU_ERR_ARG and a message from tgpu_noalloc_last_error();
  *   - the array is shared by every call and keeps the last call's contents (each call

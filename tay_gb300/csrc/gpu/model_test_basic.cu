@@ -45,9 +45,9 @@ TGPU_D void fold_fn(Seer &s, const Term &t) {
 struct See {
     using Term = test_basic::Term;
     static constexpr bool kCheapTerm = true;
-    // Candidates in flight (see pass, us): 100,000 agents 60 at 2 (an earlier walk), 41.6 at 3, 37.8
-    // at 4, 36.2 at 5, 36.1 at 6; 200,000 at eight times the pairs 454, 367, 322, 314; 30,000 27.2 at
-    // 4, 24.3 at 6.  At 8 the left-over candidates of a row cost more (46 against 43 at 4, earlier).
+    // Candidates in flight (see pass, us, at 2, 3, 4, 5, 6, 8): 100,000 agents 48.6, 40.2, 37.1,
+    // 35.5, 36.5, 39.3; 200,000 with eight times the neighbours each 353, 258, 262, 246, 248, 251;
+    // 30,000 42.2, 32.4, 28.5, 26.3, 25.4, 31.8.  At 8 the left-over candidates of a row cost more.
     static constexpr int kLaneUnroll = 6;
     static constexpr bool kSeenMinusSeer = true;  // d = b - a
     template <class Acc>

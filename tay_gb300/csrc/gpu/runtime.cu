@@ -383,8 +383,9 @@ int tgpu::prepare_specs(TgpuBatch *b) {
     b->key_bits = key_bits;
     b->specs_dirty = false;
     // box reset, bounding box (+ grids), keys and histograms (+ digit offsets), one kernel
-    // per radix pass (or one kernel for all of these, or per pass), cell table (+ reorder), the passes, and the table clear when it is
-    // a kernel (Morton order, or more segments than separate header memsets)
+    // per radix pass (or one kernel for all of these, or per pass), cell table (+ reorder), the
+    // passes, and the table clear when it is a kernel (Morton order, or more segments than
+    // separate header memsets)
     const int passes = sort_passes(b->key_bits);
     const bool clear_kernel = b->cell_order != kOrderRows || b->nseg > kMemsetClearSegments;
     const int sort = !b->cluster_blocks ? 2 + 1 + passes : b->cluster_split ? passes : 1;

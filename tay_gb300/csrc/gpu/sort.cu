@@ -131,8 +131,8 @@ __global__ void __launch_bounds__(kSortThreads) bbox_kernel(const SegmentSpec *_
     }
 }
 
-// Resets the box accumulators and the bbox kernel's block counters; a segment without agents gets its grid here, from the reset box, since no bbox block
-// runs for it.  One warp per segment.
+// Resets the box accumulators and the bbox kernel's block counters; a segment without agents
+// gets its grid here, from the reset box, since no bbox block runs for it.  One warp per segment.
 __global__ void box_reset_kernel(BoxAcc *box, uint32_t segments, const SegmentSpec *__restrict__ specs,
                                  SegGrid *__restrict__ grids, uint32_t *done) {
     const uint32_t s = (blockIdx.x * blockDim.x + threadIdx.x) / 32u;
@@ -492,11 +492,12 @@ __global__ void __launch_bounds__(kSortThreads, 4) onesweep_kernel(const Segment
 // blocks (thread-block cluster, distributed shared memory), for batches whose segments are
 // small: there the step is a chain of launches that each do next to nothing.  Box reset, box,
 // scratch memset, keys and histograms and two radix passes took 24 us of a 37 us step of
-// 2,048 agents; this launch leaves 24.6 us (12,000 agents 53 -> 40).  Every block keeps a power-of-two chunk of the segment in shared memory.  A
-// radix pass ranks the chunk stably (as onesweep_kernel), gives every block's digit counts to
-// all the others, and moves the tile's runs of equal digits to the blocks that own their
-// slots; the last pass writes keys and permutation to memory.  The same keys and a stable
-// sort: the same permutation as the general path's.
+// 2,048 agents; this launch leaves 24.6 us (12,000 agents 53 -> 40).  Every block keeps a
+// power-of-two chunk of the segment in shared memory.  A radix pass ranks the chunk stably (as
+// onesweep_kernel), gives every block's digit counts to all the others, and moves the tile's
+// runs of equal digits to the blocks that own their slots; the last pass writes keys and
+// permutation to memory.  The same keys and a stable sort: the same permutation as the general
+// path's.
 constexpr int kClusterThreads = 1024;
 constexpr int kClusterWarps = kClusterThreads / 32;
 constexpr uint32_t kClusterMost = 16;  // blocks of a cluster (above 8: opted in)

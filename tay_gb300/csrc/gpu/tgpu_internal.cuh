@@ -150,13 +150,11 @@ TGPU_HD uint32_t axis_max(const SegmentSpec &s, int i) {
 // to the cube root of the ratio).  Part-size cells hold the 27 cells around a seer's; smaller
 // ones follow its box more closely, which pays when the rows of cells are long.  Fractions
 // 1 / k, and a little more against rounding: a box of twice the part size then never touches
-// more than 2 k + 1 cells of an axis.  Measured on an SPH fluid (64 particles per cubed support
-// radius), density pass of 524,288 particles, us: 2076 at 1 (before the walk's later changes),
-// 1227 at 1/2, 1027 at 0.45, 1172 at 0.4, 1012 at 0.36, 803 at 1.004 / 3, 890 at 0.328, 833 at
-// 0.28; with the walk as it is 878 at 1/2, 746 at 1/3, 619 at 1/4, 713 at 1/5.  The force pass,
-// whose lists come out in an order with more locality, 963 at 1, 638 at 1/2, 619 at 1/3; now 525 at
-// 1/2, 491 at 1/3, 447 at 1/4.  Below some 16,000 agents the smaller cells only add radix passes
-// (2,048 particles: 53.6 us per step at 1, 61.1 at 0.34).
+// more than 2 k + 1 cells of an axis.  Measured on an SPH fluid of 524,288 particles (64 per
+// cubed support radius), us at 1, 1 / 2, 1 / 3, 1 / 4, 1 / 5 of the part size: density pass 1564,
+// 850, 738, 619, 713; force pass, whose lists come out in an order with more locality, 518, 509,
+// 496, 446, 448.  Below some 16,000 agents the smaller cells only add radix passes (2,048
+// particles: 40.0, 41.3, 44.0, 45.9 us per step at 1, 1 / 2, 1 / 3, 1 / 4).
 TGPU_HD float fill_multiple(float count, const float *ext, const float *part, int dims, float fill) {
     if (!(fill > 0.0f)) return 1.0f;
     float per_cell = count;
@@ -266,7 +264,7 @@ TGPU_HD uint32_t cell_key(const SegmentSpec &s, uint32_t x, uint32_t y, uint32_t
 // the product: 1.5 * 2^-23); a seer's interval is rounded outwards (axis_range, see.cuh).  No
 // wider than that: with cells of the see radius a seer whose interval crosses one more cell
 // border makes its whole warp walk another row of cells on each side, and a pad of 1/512 cell
-// put one in 256 seers there (see pass of 100,000 test agents 42.7 against 37.8 us).
+// puts one in 256 seers there (see pass of 100,000 test agents 39.4 against 36.5 us).
 struct SegGrid {
     Grid g;
     float pad;
